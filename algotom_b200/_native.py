@@ -15,6 +15,7 @@ LIB_PATH = os.path.join(_HERE, "lib", "libalgotom_b200.so")
 EXPORTS = ("atb_version", "atb_last_error", "atb_copy_2d", "atb_filter_length", "atb_filter_twiddles",
            "atb_filter_rows", "atb_neg_log", "atb_backproject",
            "atb_backproject_status", "atb_backproject_centers",
+           "atb_backproject_stack_workspace", "atb_backproject_stack",
            "atb_radon_workspace", "atb_radon_adjoint", "atb_bp_batch_plan",
            "atb_backproject_batch", "atb_backproject_batch_noalloc",
            "atb_gaussian_rows",
@@ -85,6 +86,12 @@ _SIGS = {
         ctypes.c_int, _vp, ctypes.c_double, ctypes.c_int, ctypes.c_double,
         ctypes.c_float, _vp, _c_i64, _c_i64, ctypes.c_int, _vp]),
     "atb_backproject_status": (ctypes.c_int, [ctypes.c_int]),
+    "atb_backproject_stack_workspace": (_c_i64, [ctypes.c_int, ctypes.c_int,
+                                                 ctypes.c_int]),
+    "atb_backproject_stack": (ctypes.c_int, [
+        _vp, ctypes.c_int, _c_i64, _c_i64, ctypes.c_int, ctypes.c_int,
+        ctypes.c_int, _vp, ctypes.c_double, ctypes.c_int, ctypes.c_double,
+        ctypes.c_float, _vp, _c_i64, _c_i64, _vp, _c_i64, _vp]),
     "atb_backproject_centers": (ctypes.c_int, [
         _vp, _c_i64, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_double,
         ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_double,

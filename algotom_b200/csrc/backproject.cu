@@ -62,6 +62,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "bp.cuh"
 #include "common.cuh"
 
 namespace {
@@ -116,6 +117,8 @@ struct BPArgs {
   int wait_polls;  // polls before a staging wait gives up (kWaitPolls)
   int inject;      // test only: CTA (0, 0, 0) arms its first staging wait
                    // for 16 bytes more than its copies deliver
+  const unsigned *gate;  // null, or ngate words (float bits): do nothing unless
+  int ngate;             // one of them is not finite
 };
 
 struct __align__(16) AngleParam {
@@ -847,6 +850,7 @@ __global__ void __launch_bounds__(BPCfg<T, S, V>::kThreads, BPCfg<T, S, V>::kMin
     bp_kernel(BPArgs a, const __grid_constant__ CUtensorMap tmap) {
   using K = BPCfg<T, S, V>;
   extern __shared__ __align__(16) unsigned char smem[];
+  if (a.gate && !__syncthreads_or((int)threadIdx.x < a.ngate && a.gate[threadIdx.x] >= 0x7f800000u)) return;
   if constexpr (kPerAngleKahan) {
     bp_tile<T, S, true, V, kGroup>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem, 0u, &tmap);
   } else {
@@ -891,6 +895,8 @@ __global__ void __launch_bounds__(BPCfg<T, 1, V>::kThreads, BPCfg<T, 1, V>::kMin
               it.sino_row_stride % 4 == 0 && it.ncol % 4 == 0;
     a.tma = 0;
     a.spacing = 0;
+    a.gate = nullptr;
+    a.ngate = 0;
     const int tiles_x = (it.ncol + K::TX - 1) / K::TX;
     bp_tile<T, 1, false, V>(a, tile % tiles_x, tile / tiles_x, 0, smem, tmem, nullptr);
   }
@@ -993,10 +999,10 @@ int dispatch(BPArgs a, int per_angle_kahan, int variant, cudaStream_t st) {
 
 }  // namespace
 
-extern "C" int atb_backproject(const void *sino, int sino_dtype, int64_t sino_row_stride, int64_t sino_slice_stride,
-                               int nrow, int nslice, int ncol, const double *trig, double center, int edge_pad,
-                               double mask_r2, float scale, float *out, int64_t out_row_stride,
-                               int64_t out_slice_stride, int flags, void *stream) {
+int atb::bp_gather(const void *sino, int sino_dtype, int64_t sino_row_stride, int64_t sino_slice_stride, int nrow,
+                   int nslice, int ncol, const double *trig, double center, int edge_pad, double mask_r2, float scale,
+                   float *out, int64_t out_row_stride, int64_t out_slice_stride, int flags, const unsigned *gate,
+                   void *stream) {
   if (!sino || !trig || !out) return atb::fail(ATB_EINVAL, "atb_backproject: null pointer");
   if (nrow < 1 || nslice < 1 || ncol < 1)
     return atb::fail(ATB_EINVAL, "atb_backproject: bad shape nrow=%d nslice=%d ncol=%d", nrow, nslice, ncol);
@@ -1017,6 +1023,8 @@ extern "C" int atb_backproject(const void *sino, int sino_dtype, int64_t sino_ro
   a.inject = (flags >> 5) & 1;
   a.wait_polls = a.inject ? 4096 : kWaitPolls;
   a.spacing = 0;
+  a.gate = gate;
+  a.ngate = nslice;
   {
     const int ve = sino_dtype == ATB_F32 ? 4 : 8;  // elements per 16-byte vector
     a.vec16 = (reinterpret_cast<uintptr_t>(sino) % 16) == 0 && sino_row_stride % ve == 0 &&
@@ -1034,7 +1042,18 @@ extern "C" int atb_backproject(const void *sino, int sino_dtype, int64_t sino_ro
   }
 }
 
+extern "C" int atb_backproject(const void *sino, int sino_dtype, int64_t sino_row_stride, int64_t sino_slice_stride,
+                               int nrow, int nslice, int ncol, const double *trig, double center, int edge_pad,
+                               double mask_r2, float scale, float *out, int64_t out_row_stride,
+                               int64_t out_slice_stride, int flags, void *stream) {
+  return atb::bp_gather(sino, sino_dtype, sino_row_stride, sino_slice_stride, nrow, nslice, ncol, trig, center,
+                        edge_pad, mask_r2, scale, out, out_row_stride, out_slice_stride, flags, nullptr, stream);
+}
+
 extern "C" int atb_backproject_status(int reset) {
+  const int mma = atb::bp_mma_status(reset);
+  if (mma < 0)
+    return atb::fail(ATB_ECUDA, "atb_backproject_status: %s", cudaGetErrorString(cudaGetLastError()));
   int v = 0;
   if (cudaMemcpyFromSymbol(&v, g_bp_status, sizeof(int)) != cudaSuccess)
     return atb::fail(ATB_ECUDA, "atb_backproject_status: %s", cudaGetErrorString(cudaGetLastError()));
@@ -1043,7 +1062,7 @@ extern "C" int atb_backproject_status(int reset) {
     if (cudaMemcpyToSymbol(g_bp_status, &zero, sizeof(int)) != cudaSuccess)
       return atb::fail(ATB_ECUDA, "atb_backproject_status: %s", cudaGetErrorString(cudaGetLastError()));
   }
-  return v;
+  return v | mma;
 }
 
 extern "C" int atb_backproject_centers(const float *sino, int64_t sino_row_stride, int nrow, int ncol,
@@ -1078,6 +1097,8 @@ extern "C" int atb_backproject_centers(const float *sino, int64_t sino_row_strid
   a.inject = 0;
   a.wait_polls = kWaitPolls;
   a.spacing = spacing;
+  a.gate = nullptr;
+  a.ngate = 0;
   a.vec16 = (reinterpret_cast<uintptr_t>(sino) % 16) == 0 && sino_row_stride % 4 == 0 && ncol % 4 == 0;
   cudaStream_t st = atb::as_stream(stream);
   // four centres per CTA, then the remainder

@@ -165,7 +165,9 @@ def backproject(sino3, angles, center, edge_pad=False, mask_r2=-1.0,
     the single-slice tile variant (0: 64 x 64, 1: 32 x 32).  ``staging``:
     "tma" stages the detector windows of 2- and 4-slice CTAs with TMA box
     loads where the rows are 16-byte aligned, "cp.async" always with
-    cp.async; the results are the same.
+    cp.async; the results are the same.  Stacks of 15 and more slices run on
+    the tensor cores (``atb_backproject_stack``) unless ``kahan`` is "angle"
+    or ``staging`` "cp.async".
     """
     if staging not in ("tma", "cp.async"):
         raise ValueError("staging must be 'tma' or 'cp.async'")
@@ -178,6 +180,18 @@ def backproject(sino3, angles, center, edge_pad=False, mask_r2=-1.0,
     if out is None:
         out = torch.empty((ncol, nslice, ncol), dtype=torch.float32,
                           device=dev)
+    if kahan != "angle" and staging == "tma":
+        need = nat.call("atb_backproject_stack_workspace", nrow, nslice, ncol)
+        if need > 0:
+            ws = _stack_workspace(need, dev)
+            nat.call("atb_backproject_stack", sino3.data_ptr(), code,
+                     sino3.stride(0), sino3.stride(1), nrow, nslice, ncol,
+                     trig.data_ptr(), float(np.float32(center)),
+                     int(bool(edge_pad)), float(mask_r2), float(scale),
+                     out.data_ptr(), out.stride(0), out.stride(1),
+                     ws.data_ptr() if ws is not None else None,
+                     need if ws is not None else 0, _stream_ptr(dev))
+            return out
     nat.call("atb_backproject", sino3.data_ptr(), code, sino3.stride(0),
              sino3.stride(1), nrow, nslice, ncol, trig.data_ptr(),
              float(np.float32(center)), int(bool(edge_pad)), float(mask_r2),
@@ -185,6 +199,16 @@ def backproject(sino3, angles, center, edge_pad=False, mask_r2=-1.0,
              (1 if kahan == "angle" else 0) | (int(variant) << 2) |
              (16 if staging == "cp.async" else 0), _stream_ptr(dev))
     return out
+
+
+def _stack_workspace(nbytes, device):
+    """Device scratch of the tensor-core back-projector (freed in stream
+    order by the caching allocator); None where the memory is not there, and
+    the stack takes the gather kernel, which needs none."""
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None
 
 
 def _backproject_tuned(f, angles, center, **kw):
