@@ -86,12 +86,12 @@ _SIGS = {
         ctypes.c_int, _vp, ctypes.c_double, ctypes.c_int, ctypes.c_double,
         ctypes.c_float, _vp, _c_i64, _c_i64, ctypes.c_int, _vp]),
     "atb_backproject_status": (ctypes.c_int, [ctypes.c_int]),
-    "atb_backproject_stack_workspace": (_c_i64, [ctypes.c_int, ctypes.c_int,
-                                                 ctypes.c_int]),
+    "atb_backproject_stack_workspace": (_c_i64, [
+        ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     "atb_backproject_stack": (ctypes.c_int, [
         _vp, ctypes.c_int, _c_i64, _c_i64, ctypes.c_int, ctypes.c_int,
         ctypes.c_int, _vp, ctypes.c_double, ctypes.c_int, ctypes.c_double,
-        ctypes.c_float, _vp, _c_i64, _c_i64, _vp, _c_i64, _vp]),
+        ctypes.c_float, _vp, _c_i64, _c_i64, ctypes.c_int, _vp, _c_i64, _vp]),
     "atb_backproject_centers": (ctypes.c_int, [
         _vp, _c_i64, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_double,
         ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_double,

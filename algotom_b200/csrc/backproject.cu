@@ -58,6 +58,7 @@
 #include <cuda.h>  // CUtensorMap and its enums (the encoder is fetched at run time)
 #include <cudaTypedefs.h>
 
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
@@ -119,7 +120,15 @@ struct BPArgs {
                    // for 16 bytes more than its copies deliver
   const unsigned *gate;  // null, or ngate words (float bits): do nothing unless
   int ngate;             // one of them is not finite
+  // angle groups: CTA layer g of ngroup walks the angles from g * group_rows
+  // and leaves its compensated totals, not pixels, in part
+  // [ngroup][nslice][ncol][ncol] (total, compensation)
+  int ngroup, group_rows;
+  int row0;  // first angle of this CTA's group
+  float2 *part;
 };
+
+__device__ __forceinline__ long long ncol2(int ncol) { return (long long)ncol * ncol; }
 
 struct __align__(16) AngleParam {
   float qbase;  // local position of the tile-origin pixel, q = p - lo - H
@@ -367,6 +376,22 @@ __device__ __forceinline__ void bp_tile(const BPArgs &a, int bx, int by, int bz,
   const int nsl = min(S, a.nslice - slice0);  // live slices of this CTA
   const bool use_tma = a.tma != 0;
   const int ncol = a.ncol;
+  // a tile wholly outside the circle mask is zero (with angle groups the
+  // reduction writes it)
+  if (a.mask_r2 >= 0.0) {
+    const int cm = ncol / 2;
+    const long long dx = max(0, max(x0 - cm, cm - (x0 + TX - 1))), dy = max(0, max(y0 - cm, cm - (y0 + TY - 1)));
+    if ((double)(dx * dx + dy * dy) > a.mask_r2) {
+      if (!a.part) {
+        for (int e = tid; e < TX * TY; e += kThreads) {
+          const int x = x0 + e % TX, y = y0 + e / TX;
+          if (x < ncol && y < ncol)
+            for (int k = 0; k < nsl; ++k) a.out[y * a.ors + (slice0 + k) * a.oss + x] = 0.f;
+        }
+      }
+      return;
+    }
+  }
   const T *sino = reinterpret_cast<const T *>(a.sino) + slice0 * a.sss;
   // centre-group launches: this CTA's first centre, the shift between its
   // slices and the length of the row segment it stages
@@ -492,7 +517,7 @@ __device__ __forceinline__ void bp_tile(const BPArgs &a, int bx, int by, int bz,
         unsigned bytes = (unsigned)(kGroup ? seglen * (int)sizeof(T) : K::kBoxBytes);
         if (a.inject && k == 0 && tid == 0 && bx == 0 && by == 0 && bz == 0) bytes += 16u;
         mbar_arrive_expect_tx(&raw_bar, bytes);
-        tma_load_3d(raw + (size_t)tid * K::kRawSlot, tmap, base, kGroup ? 0 : slice0, it, &raw_bar);
+        tma_load_3d(raw + (size_t)tid * K::kRawSlot, tmap, base, kGroup ? 0 : slice0, a.row0 + it, &raw_bar);
       } else {
         mbar_arrive(&raw_bar);
       }
@@ -835,7 +860,9 @@ __device__ __forceinline__ void bp_tile(const BPArgs &a, int bx, int by, int bz,
         }
 #pragma unroll
         for (int k = 0; k < S; ++k) {
-          if (k < nsl) {
+          if (k < nsl && a.part) {
+            a.part[((long long)(slice0 + k) * ncol + y) * ncol + x] = make_float2(sum[b][c][k], comp[b][c][k]);
+          } else if (k < nsl) {
             const float v = keep ? __fsub_rn(sum[b][c][k], comp[b][c][k]) * a.scale : 0.f;
             a.out[y * a.ors + (slice0 + k) * a.oss + x] = v;
           }
@@ -851,12 +878,22 @@ __global__ void __launch_bounds__(BPCfg<T, S, V>::kThreads, BPCfg<T, S, V>::kMin
   using K = BPCfg<T, S, V>;
   extern __shared__ __align__(16) unsigned char smem[];
   if (a.gate && !__syncthreads_or((int)threadIdx.x < a.ngate && a.gate[threadIdx.x] >= 0x7f800000u)) return;
+  int bz = blockIdx.z;
+  if (a.part) {  // this CTA's angle group
+    const int nz = gridDim.z / a.ngroup, g = bz / nz;
+    bz -= g * nz;
+    a.row0 = g * a.group_rows;
+    a.sino = reinterpret_cast<const T *>(a.sino) + a.row0 * a.srs;
+    a.trig += a.row0;
+    a.nrow = min(a.group_rows, a.nrow - a.row0);
+    a.part += (long long)g * a.nslice * ncol2(a.ncol);
+  }
   if constexpr (kPerAngleKahan) {
-    bp_tile<T, S, true, V, kGroup>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem, 0u, &tmap);
+    bp_tile<T, S, true, V, kGroup>(a, blockIdx.x, blockIdx.y, bz, smem, 0u, &tmap);
   } else {
     __shared__ uint32_t tmem_slot;
     const uint32_t tmem = tmem_alloc_cta<K::kTmemCols>(&tmem_slot);
-    bp_tile<T, S, false, V, kGroup>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem, tmem, &tmap);
+    bp_tile<T, S, false, V, kGroup>(a, blockIdx.x, blockIdx.y, bz, smem, tmem, &tmap);
     tmem_free_cta<K::kTmemCols>(tmem);
   }
 }
@@ -897,6 +934,9 @@ __global__ void __launch_bounds__(BPCfg<T, 1, V>::kThreads, BPCfg<T, 1, V>::kMin
     a.spacing = 0;
     a.gate = nullptr;
     a.ngate = 0;
+    a.ngroup = 1;
+    a.row0 = 0;
+    a.part = nullptr;
     const int tiles_x = (it.ncol + K::TX - 1) / K::TX;
     bp_tile<T, 1, false, V>(a, tile % tiles_x, tile / tiles_x, 0, smem, tmem, nullptr);
   }
@@ -959,8 +999,58 @@ bool make_window_map(const BPArgs &a, CUtensorMap *map) {
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Pixels from the angle groups' totals: their exact sum in FP64, rounded once,
+// mask, scale.
+__global__ void __launch_bounds__(256) sum_groups_kernel(BPArgs a) {
+  const long long total = (long long)a.nslice * a.ncol * a.ncol;
+  const int cm = a.ncol / 2;
+  for (long long e = blockIdx.x * 256ll + threadIdx.x; e < total; e += gridDim.x * 256ll) {
+    const int x = (int)(e % a.ncol);
+    const long long t = e / a.ncol;
+    const int y = (int)(t % a.ncol), k = (int)(t / a.ncol);
+    float v = 0.f;
+    const long long dx = x - cm, dy = y - cm;
+    if (a.mask_r2 < 0.0 || (double)(dx * dx + dy * dy) <= a.mask_r2) {
+      double s = 0.0;
+      for (int g = 0; g < a.ngroup; ++g) {
+        const float2 p = a.part[g * total + e];
+        s += (double)p.x - (double)p.y;
+      }
+      v = (float)s * a.scale;
+    }
+    a.out[y * a.ors + k * a.oss + x] = v;
+  }
+}
+
+// Angles per CTA when a launch's tiles do not fill the GPU evenly: nrow (no
+// groups), or a multiple of the chunk.  A wave of CTAs takes as long as its
+// angles and about 40 more (prologue, epilogue); the sum of n groups' partial
+// images costs their traffic and a launch, in units of the 0.3 us that a wave
+// takes for an angle.  Tiles outside the inscribed disc are counted as empty
+// (they are with the default mask).
+template <typename T, int S, int V>
+int group_rows(int nrow, int nslices, int ncol) {
+  using K = BPCfg<T, S, V>;
+  const double tiles = 0.785 * ((ncol + K::TX - 1) / K::TX) * (double)((ncol + K::TY - 1) / K::TY) * ((nslices + S - 1) / S);
+  const double slots = 148.0 * K::kMinBlocks;
+  const int nchunk = (nrow + K::kChunk - 1) / K::kChunk;
+  double best = 0.0;
+  int rows = nrow;
+  for (int g = 1; g <= 32 && g <= nchunk; ++g) {
+    const int r = (nchunk + g - 1) / g * K::kChunk, n = (nrow + r - 1) / r;
+    if (g > 1 && n != g) continue;
+    double cost = ceil(tiles * n / slots) * ((n > 1 ? r : nrow) + 40.0);
+    if (n > 1) cost += 13.0 + (double)ncol * ncol * nslices * n * 16.0 / 1.2e6;
+    if (g == 1 || cost < 0.95 * best) {
+      best = cost;
+      rows = n > 1 ? r : nrow;
+    }
+  }
+  return rows;
+}
+
 template <typename T, int S, bool kPerAngleKahan, int V = 0, bool kGroup = false>
-int launch_bp(BPArgs a, int nslices, cudaStream_t st) {
+int launch_bp(BPArgs a, int nslices, cudaStream_t st, float2 *work = nullptr) {
   using K = BPCfg<T, S, V>;
   auto fn = bp_kernel<T, S, kPerAngleKahan, V, kGroup>;
   const int rc = atb::ensure_smem(fn, K::kSmem, "atb_backproject", K::kThreads, kPerAngleKahan ? 0 : K::kTmemCols);
@@ -972,29 +1062,69 @@ int launch_bp(BPArgs a, int nslices, cudaStream_t st) {
   // does not speed up, so they keep cp.async
   a.tma = a.tma && S >= 2 && make_window_map<T, S, V, kGroup>(a, &map);
   dim3 grid((a.ncol + K::TX - 1) / K::TX, (a.ncol + K::TY - 1) / K::TY, (nslices + S - 1) / S);
+  a.ngroup = 1;
+  a.row0 = 0;
+  a.part = nullptr;
+  if (work) {
+    const int rows = group_rows<T, S, V>(a.nrow, nslices, a.ncol);
+    if (rows < a.nrow) {
+      a.group_rows = rows;
+      a.ngroup = (a.nrow + rows - 1) / rows;
+      a.part = work;
+      // the partial images hold this launch's slices only
+      a.sino = static_cast<const T *>(a.sino) + a.slice_base * a.sss;
+      a.out += a.slice_base * a.oss;
+      a.slice_base = 0;
+      a.nslice = nslices;
+      if (a.tma) a.tma = make_window_map<T, S, V, kGroup>(a, &map);
+      grid.z *= a.ngroup;
+    }
+  }
   fn<<<grid, K::kThreads, K::kSmem, st>>>(a, map);
-  return atb::check_launch("atb_backproject");
+  const int rcl = atb::check_launch("atb_backproject");
+  if (rcl != ATB_OK || !a.part) return rcl;
+  const long long total = (long long)nslices * a.ncol * a.ncol;
+  const long long blocks = (total + 255) / 256;
+  sum_groups_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, st>>>(a);
+  return atb::check_launch("atb_backproject (angle groups)");
 }
 
+// work: null, or scratch for the angle groups (split_bytes)
 template <typename T>
-int dispatch(BPArgs a, int per_angle_kahan, int variant, cudaStream_t st) {
+int dispatch(BPArgs a, int per_angle_kahan, int variant, cudaStream_t st, float2 *work) {
   if (per_angle_kahan) return launch_bp<T, 1, true>(a, a.nslice, st);
-  if (a.nslice == 1 && variant == 1) return launch_bp<T, 1, false, 1>(a, 1, st);
+  if (work) variant = 1;  // (the smaller tiles split better)
+  if (a.nslice == 1 && variant == 1) return launch_bp<T, 1, false, 1>(a, 1, st, work);
   // four slices per CTA for the bulk of a stack, then the remainder
   const int n4 = (a.nslice / 4) * 4;
   int rc = ATB_OK;
-  if (n4 > 0) rc = launch_bp<T, 4, false>(a, n4, st);
+  if (n4 > 0) rc = launch_bp<T, 4, false>(a, n4, st, work);
   if (rc != ATB_OK) return rc;
   const int rem = a.nslice - n4;
   if (rem == 0) return ATB_OK;
   a.slice_base = n4;
   if (rem >= 2) {
-    rc = launch_bp<T, 2, false>(a, 2, st);
+    rc = launch_bp<T, 2, false>(a, 2, st, work);
     if (rc != ATB_OK || rem == 2) return rc;
     a.slice_base = n4 + 2;
   }
-  if (variant == 1) return launch_bp<T, 1, false, 1>(a, 1, st);
+  if (variant == 1) return launch_bp<T, 1, false, 1>(a, 1, st, work);
   return launch_bp<T, 1, false>(a, 1, st);
+}
+
+// bytes of the partial images of dispatch's largest launch; 0 without groups
+template <typename T>
+long long split_bytes(int nrow, int nslice, int ncol) {
+  long long need = 0;
+  auto add = [&](int rows, int n) {
+    const long long groups = (nrow + rows - 1) / rows;
+    if (groups > 1 && groups * n * ncol * (long long)ncol * 8 > need) need = groups * n * ncol * (long long)ncol * 8;
+  };
+  const int n4 = (nslice / 4) * 4, rem = nslice - n4;
+  if (n4 > 0) add(group_rows<T, 4, 0>(nrow, n4, ncol), n4);
+  if (rem >= 2) add(group_rows<T, 2, 0>(nrow, 2, ncol), 2);
+  if (rem & 1) add(group_rows<T, 1, 1>(nrow, 1, ncol), 1);
+  return need;
 }
 
 }  // namespace
@@ -1002,7 +1132,7 @@ int dispatch(BPArgs a, int per_angle_kahan, int variant, cudaStream_t st) {
 int atb::bp_gather(const void *sino, int sino_dtype, int64_t sino_row_stride, int64_t sino_slice_stride, int nrow,
                    int nslice, int ncol, const double *trig, double center, int edge_pad, double mask_r2, float scale,
                    float *out, int64_t out_row_stride, int64_t out_slice_stride, int flags, const unsigned *gate,
-                   void *stream) {
+                   void *work, void *stream) {
   if (!sino || !trig || !out) return atb::fail(ATB_EINVAL, "atb_backproject: null pointer");
   if (nrow < 1 || nslice < 1 || ncol < 1)
     return atb::fail(ATB_EINVAL, "atb_backproject: bad shape nrow=%d nslice=%d ncol=%d", nrow, nslice, ncol);
@@ -1035,9 +1165,9 @@ int atb::bp_gather(const void *sino, int sino_dtype, int64_t sino_row_stride, in
   const int variant = (flags >> 2) & 3;
   if (variant > 1) return atb::fail(ATB_EINVAL, "atb_backproject: unknown tile variant %d", variant);
   switch (sino_dtype) {
-    case ATB_F32: return dispatch<float>(a, pak, variant, st);
-    case ATB_F16: return dispatch<__half>(a, pak, variant, st);
-    case ATB_BF16: return dispatch<__nv_bfloat16>(a, pak, variant, st);
+    case ATB_F32: return dispatch<float>(a, pak, variant, st, static_cast<float2 *>(work));
+    case ATB_F16: return dispatch<__half>(a, pak, variant, st, static_cast<float2 *>(work));
+    case ATB_BF16: return dispatch<__nv_bfloat16>(a, pak, variant, st, static_cast<float2 *>(work));
     default: return atb::fail(ATB_EINVAL, "atb_backproject: unknown sino_dtype %d", sino_dtype);
   }
 }
@@ -1047,7 +1177,12 @@ extern "C" int atb_backproject(const void *sino, int sino_dtype, int64_t sino_ro
                                double mask_r2, float scale, float *out, int64_t out_row_stride,
                                int64_t out_slice_stride, int flags, void *stream) {
   return atb::bp_gather(sino, sino_dtype, sino_row_stride, sino_slice_stride, nrow, nslice, ncol, trig, center,
-                        edge_pad, mask_r2, scale, out, out_row_stride, out_slice_stride, flags, nullptr, stream);
+                        edge_pad, mask_r2, scale, out, out_row_stride, out_slice_stride, flags, nullptr, nullptr, stream);
+}
+
+long long atb::bp_gather_workspace(int nrow, int nslice, int ncol) {
+  // (the sample type changes no tile or chunk)
+  return split_bytes<float>(nrow, nslice, ncol);
 }
 
 extern "C" int atb_backproject_status(int reset) {
@@ -1099,6 +1234,9 @@ extern "C" int atb_backproject_centers(const float *sino, int64_t sino_row_strid
   a.spacing = spacing;
   a.gate = nullptr;
   a.ngate = 0;
+  a.ngroup = 1;
+  a.row0 = 0;
+  a.part = nullptr;
   a.vec16 = (reinterpret_cast<uintptr_t>(sino) % 16) == 0 && sino_row_stride % 4 == 0 && ncol % 4 == 0;
   cudaStream_t st = atb::as_stream(stream);
   // four centres per CTA, then the remainder

@@ -8,11 +8,13 @@ namespace atb {
 // The gather back-projector behind atb_backproject (same arguments).  gate:
 // null, or a device array of nslice words, the float bits of each slice's
 // largest magnitude: the launch does its work only if one of them is not
-// finite.
+// finite.  work: null, or scratch of bp_gather_workspace bytes, with which
+// launches whose tiles do not fill the GPU split the angles over more CTAs.
 int bp_gather(const void *sino, int sino_dtype, int64_t sino_row_stride, int64_t sino_slice_stride, int nrow,
               int nslice, int ncol, const double *trig, double center, int edge_pad, double mask_r2, float scale,
               float *out, int64_t out_row_stride, int64_t out_slice_stride, int flags, const unsigned *gate,
-              void *stream);
+              void *work, void *stream);
+long long bp_gather_workspace(int nrow, int nslice, int ncol);  // 0: none is used
 
 // Status word of the tensor-core back-projector, as atb_backproject_status.
 int bp_mma_status(int reset);

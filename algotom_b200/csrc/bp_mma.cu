@@ -754,8 +754,11 @@ int prepare(const void *sino, long long srs, long long sss, int nrow, int nsl, i
 // slices of the next launch of a stack with n left: 0 if the gather kernel is
 // the faster one for all of them.  A launch costs the same for 16 as for 10
 // slices, at 901 x 1280 6.1 ms, and the gather kernel 0.43 ms per slice: 6.0
-// for 14, 6.5 for 15.
-int next_group(int n) {
+// for 14, 6.5 for 15.  bfloat16 samples stay with the gather kernel, whose
+// interpolation differences are bfloat16 too: a user's results would move by
+// that rounding (2e-4) for a faster kernel.
+int next_group(int sino_dtype, int n) {
+  if (sino_dtype == ATB_BF16) return 0;
   if (n >= 32) return 32;
   return n >= 15 ? n : 0;
 }
@@ -775,36 +778,39 @@ int bp_mma_status(int reset) {
 }
 }  // namespace atb
 
-extern "C" int64_t atb_backproject_stack_workspace(int nrow, int nslice, int ncol) {
+extern "C" int64_t atb_backproject_stack_workspace(int sino_dtype, int nrow, int nslice, int ncol) {
   if (nrow < 1 || nslice < 1 || ncol < 1 || nrow > 65535 || ncol > (1 << 16)) return 0;
-  const int n = next_group(nslice);
-  if (n == 0) return 0;
-  return kHeader + (int64_t)nrow * ncol * padded(n) * 4;
+  const int n = next_group(sino_dtype, nslice);
+  const int64_t packed = n ? kHeader + (int64_t)nrow * ncol * padded(n) * 4 : 0;
+  // slices left over after the last launch of the tensor cores
+  int left = nslice;
+  if (n == 32) left %= 32;
+  if (next_group(sino_dtype, left)) left = 0;
+  const int64_t split = left ? atb::bp_gather_workspace(nrow, left, ncol) : 0;
+  return packed > split ? packed : split;
 }
 
 extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t sino_row_stride,
                                      int64_t sino_slice_stride, int nrow, int nslice, int ncol, const double *trig,
                                      double center, int edge_pad, double mask_r2, float scale, float *out,
-                                     int64_t out_row_stride, int64_t out_slice_stride, void *workspace,
+                                     int64_t out_row_stride, int64_t out_slice_stride, int flags, void *workspace,
                                      int64_t workspace_bytes, void *stream) {
+  if (flags & ~16) return atb::fail(ATB_EINVAL, "atb_backproject_stack: unknown flags %d", flags);
   cudaStream_t st = atb::as_stream(stream);
-  const int64_t need = atb_backproject_stack_workspace(nrow, nslice, ncol);
+  const int64_t need = atb_backproject_stack_workspace(sino_dtype, nrow, nslice, ncol);
   const int esize = sino_dtype == ATB_F32 ? 4 : 2;
   int first = 0;
+  const bool work_ok = need > 0 && workspace && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 128 == 0;
   const bool args_ok = sino && trig && out && (sino_dtype == ATB_F32 || sino_dtype == ATB_F16 || sino_dtype == ATB_BF16) &&
                        center >= 0.0 && center < (double)ncol;
-  if (args_ok && need > 0 && workspace && workspace_bytes >= need &&
-      reinterpret_cast<uintptr_t>(workspace) % 128 == 0) {
-    for (int n; (n = next_group(nslice - first)) > 0; first += n) {
+  if (args_ok && work_ok) {
+    for (int n; (n = next_group(sino_dtype, nslice - first)) > 0; first += n) {
       const int S = padded(n);
       const char *src = static_cast<const char *>(sino) + (int64_t)first * sino_slice_stride * esize;
       float *dst = out + (int64_t)first * out_slice_stride;
-      int rc;
-      switch (sino_dtype) {
-        case ATB_F32: rc = prepare<float>(src, sino_row_stride, sino_slice_stride, nrow, n, ncol, S, workspace, st); break;
-        case ATB_F16: rc = prepare<__half>(src, sino_row_stride, sino_slice_stride, nrow, n, ncol, S, workspace, st); break;
-        default: rc = prepare<__nv_bfloat16>(src, sino_row_stride, sino_slice_stride, nrow, n, ncol, S, workspace, st); break;
-      }
+      int rc = sino_dtype == ATB_F32
+                   ? prepare<float>(src, sino_row_stride, sino_slice_stride, nrow, n, ncol, S, workspace, st)
+                   : prepare<__half>(src, sino_row_stride, sino_slice_stride, nrow, n, ncol, S, workspace, st);
       if (rc != ATB_OK) return rc;
       MmaArgs a;
       a.maxbits = static_cast<const unsigned *>(workspace);
@@ -824,7 +830,7 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
       if (rc != ATB_OK) return rc;
       // runs only where a sample is not finite
       rc = atb::bp_gather(src, sino_dtype, sino_row_stride, sino_slice_stride, nrow, n, ncol, trig, center, edge_pad,
-                          mask_r2, scale, dst, out_row_stride, out_slice_stride, 0, a.maxbits, stream);
+                          mask_r2, scale, dst, out_row_stride, out_slice_stride, flags, a.maxbits, nullptr, stream);
       if (rc != ATB_OK) return rc;
     }
     if (first == nslice) return ATB_OK;
@@ -832,5 +838,5 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
   return atb::bp_gather(args_ok ? static_cast<const char *>(sino) + (int64_t)first * sino_slice_stride * esize : sino,
                         sino_dtype, sino_row_stride, sino_slice_stride, nrow, nslice - first, ncol, trig, center,
                         edge_pad, mask_r2, scale, out ? out + (int64_t)first * out_slice_stride : out, out_row_stride,
-                        out_slice_stride, 0, nullptr, stream);
+                        out_slice_stride, flags, nullptr, work_ok ? workspace : nullptr, stream);
 }

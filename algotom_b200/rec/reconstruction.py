@@ -15,6 +15,7 @@ memory), ``storage`` ("float32", "float16" or "bfloat16": the element type
 of the filtered sinogram between the two kernels) and ``kahan`` ("chunk",
 the default, or "angle").
 """
+import functools
 import math
 import warnings
 
@@ -26,6 +27,8 @@ from . import windows as win
 from .windows import (make_smoothing_window, make_2d_ramp_window,  # noqa: F401
                       make_circular_ramp_window)
 
+_CODES = {torch.float32: nat.F32, torch.float16: nat.F16,
+          torch.bfloat16: nat.BF16}
 _STORAGE = {"float32": (torch.float32, nat.F32),
             "float16": (torch.float16, nat.F16),
             "bfloat16": (torch.bfloat16, nat.BF16)}
@@ -165,23 +168,23 @@ def backproject(sino3, angles, center, edge_pad=False, mask_r2=-1.0,
     the single-slice tile variant (0: 64 x 64, 1: 32 x 32).  ``staging``:
     "tma" stages the detector windows of 2- and 4-slice CTAs with TMA box
     loads where the rows are 16-byte aligned, "cp.async" always with
-    cp.async; the results are the same.  Stacks of 15 and more slices run on
-    the tensor cores (``atb_backproject_stack``) unless ``kahan`` is "angle"
-    or ``staging`` "cp.async".
+    cp.async; the results are the same.  Unless ``kahan`` is "angle", stacks
+    of 15 and more slices (not bfloat16) run on the tensor cores, and launches
+    with few tiles split the angles over more CTAs, ``variant`` or not
+    (``atb_backproject_stack``).
     """
     if staging not in ("tma", "cp.async"):
         raise ValueError("staging must be 'tma' or 'cp.async'")
     nrow, nslice, ncol = sino3.shape
     dev = sino3.device
-    code = {torch.float32: nat.F32, torch.float16: nat.F16,
-            torch.bfloat16: nat.BF16}[sino3.dtype]
+    code = _CODES[sino3.dtype]
     if trig is None:
         trig = _trig(angles, dev)
     if out is None:
         out = torch.empty((ncol, nslice, ncol), dtype=torch.float32,
                           device=dev)
-    if kahan != "angle" and staging == "tma":
-        need = nat.call("atb_backproject_stack_workspace", nrow, nslice, ncol)
+    if kahan != "angle":
+        need = _stack_need(code, nrow, nslice, ncol)
         if need > 0:
             ws = _stack_workspace(need, dev)
             nat.call("atb_backproject_stack", sino3.data_ptr(), code,
@@ -189,6 +192,7 @@ def backproject(sino3, angles, center, edge_pad=False, mask_r2=-1.0,
                      trig.data_ptr(), float(np.float32(center)),
                      int(bool(edge_pad)), float(mask_r2), float(scale),
                      out.data_ptr(), out.stride(0), out.stride(1),
+                     16 if staging == "cp.async" else 0,
                      ws.data_ptr() if ws is not None else None,
                      need if ws is not None else 0, _stream_ptr(dev))
             return out
@@ -201,10 +205,18 @@ def backproject(sino3, angles, center, edge_pad=False, mask_r2=-1.0,
     return out
 
 
+@functools.lru_cache(maxsize=256)
+def _stack_need(code, nrow, nslice, ncol):
+    """Scratch bytes of ``atb_backproject_stack`` (a rule on the sizes); 0
+    where it is ``atb_backproject``."""
+    return nat.call("atb_backproject_stack_workspace", code, nrow, nslice,
+                    ncol)
+
+
 def _stack_workspace(nbytes, device):
-    """Device scratch of the tensor-core back-projector (freed in stream
-    order by the caching allocator); None where the memory is not there, and
-    the stack takes the gather kernel, which needs none."""
+    """Scratch of ``atb_backproject_stack`` (freed in stream order by the
+    caching allocator); None where the memory is not there: the call then is
+    ``atb_backproject``, which needs none."""
     try:
         return torch.empty(nbytes, dtype=torch.uint8, device=device)
     except torch.OutOfMemoryError:
@@ -215,7 +227,8 @@ def _backproject_tuned(f, angles, center, **kw):
     """Back-projection of a single slice with the autotuned tile variant."""
     from .autotune import tuned_single_variant
     nrow, nslice, ncol = f.shape
-    if nslice != 1 or kw.get("kahan") == "angle":
+    if nslice != 1 or kw.get("kahan") == "angle" or \
+            _stack_need(_CODES[f.dtype], nrow, 1, ncol) > 0:
         return backproject(f, angles, center, **kw)
     trig = _trig(angles, f.device)
     out = torch.empty((ncol, 1, ncol), dtype=torch.float32, device=f.device)

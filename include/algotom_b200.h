@@ -214,26 +214,30 @@ int atb_backproject(const void *sino, int sino_dtype, int64_t sino_row_stride,
                     int flags, void *stream);
 
 /*
- * atb_backproject (with flags 0) of a stack, given a workspace: stacks of 15
- * and more slices run on the tensor cores, up to 32 slices per launch, what
- * is left over and every stack without a (large enough) workspace as
- * atb_backproject does.  Samples and weights are split in two float16 terms
- * each and the sums are compensated FP32: results differ from
- * atb_backproject's by rounding only.  Stacks with non-finite samples give
- * atb_backproject's results.
+ * atb_backproject, given a workspace.  Stacks of 15 and more
+ * float32 or float16 slices run on the tensor cores, up to 32 slices per
+ * launch: samples and weights are split in two float16 terms each and the sums
+ * are compensated FP32, so that results differ from atb_backproject's by
+ * rounding only; stacks with non-finite samples give atb_backproject's
+ * results.  Launches whose tiles do not fill the GPU split the angles over
+ * more CTAs and add the parts in FP64.  Everything else, and every call
+ * without a (large enough) workspace, is atb_backproject.
  *
+ *   flags      bit 4 as atb_backproject (the same results), else 0
  *   workspace  128-byte aligned device scratch of
  *              atb_backproject_stack_workspace bytes (0: none is used), free
  *              for reuse when the call's work on the stream is done
  */
-int64_t atb_backproject_stack_workspace(int nrow, int nslice, int ncol);
+int64_t atb_backproject_stack_workspace(int sino_dtype, int nrow, int nslice,
+                                        int ncol);
 int atb_backproject_stack(const void *sino, int sino_dtype,
                           int64_t sino_row_stride, int64_t sino_slice_stride,
                           int nrow, int nslice, int ncol, const double *trig,
                           double center, int edge_pad, double mask_r2,
                           float scale, float *out, int64_t out_row_stride,
-                          int64_t out_slice_stride, void *workspace,
-                          int64_t workspace_bytes, void *stream);
+                          int64_t out_slice_stride, int flags,
+                          void *workspace, int64_t workspace_bytes,
+                          void *stream);
 
 /*
  * Back-projection of ONE sinogram at ncenter rotation centres

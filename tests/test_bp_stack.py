@@ -25,6 +25,18 @@ def _stack(nrow, nslice, ncol, seed=0):
     return x * 10.0 ** rng.integers(-3, 4, (1, nslice, 1)).astype(np.float32)
 
 
+def _gather(t, ang, cen, edge_pad=False):
+    """``atb_backproject`` itself: no tensor cores, no angle groups."""
+    nrow, nslice, ncol = t.shape
+    out = torch.empty((ncol, nslice, ncol), device=t.device)
+    nat.call("atb_backproject", t.data_ptr(), nat.F32, t.stride(0),
+             t.stride(1), nrow, nslice, ncol,
+             R._trig(ang, t.device).data_ptr(), float(np.float32(cen)),
+             int(edge_pad), -1.0, 1.0, out.data_ptr(), out.stride(0),
+             out.stride(1), 0, R._stream_ptr(t.device))
+    return out
+
+
 def _check(x, ang, cen, edge_pad, cuda, **kw):
     got = R.backproject(torch.from_numpy(x).to(cuda), ang, cen,
                         edge_pad=edge_pad, **kw).cpu().numpy()
@@ -41,18 +53,22 @@ def _check(x, ang, cen, edge_pad, cuda, **kw):
     (8, 25, 31, 30.0), (9, 31, 33, 16.0), (16, 32, 48, 20.7),
     (17, 33, 40, 19.5), (33, 47, 65, 33.3), (40, 64, 100, 12.1)])
 def test_stack_against_oracle(cuda, nrow, nslice, ncol, cen, edge_pad):
-    assert nat.call("atb_backproject_stack_workspace", nrow, nslice, ncol) > 0
+    assert nat.call("atb_backproject_stack_workspace", nat.F32, nrow, nslice,
+                    ncol) > 0
     ang = np.linspace(0.0, np.pi, nrow)  # 0, 90 and 180 degrees among them
     _check(_stack(nrow, nslice, ncol, nrow), ang, cen, edge_pad, cuda)
 
 
 def test_small_stacks_take_the_gather_kernel():
-    assert nat.call("atb_backproject_stack_workspace", 181, 14, 256) == 0
-    assert nat.call("atb_backproject_stack_workspace", 181, 15, 256) > 0
+    def need(code, nslice):
+        return nat.call("atb_backproject_stack_workspace", code, 181, nslice,
+                        2560)
+    assert need(nat.F32, 14) == need(nat.BF16, 32) == 0
+    assert need(nat.F32, 15) > 0 and need(nat.F16, 15) > 0
 
 
-@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-def test_stack_of_16_bit_samples_with_mask_and_strides(cuda, dtype):
+def test_stack_of_16_bit_samples_with_mask_and_strides(cuda):
+    dtype = torch.float16
     nrow, nslice, ncol = 21, 18, 50
     x = torch.from_numpy(_stack(nrow, nslice, ncol)).clamp(1e-3, 1e3)
     wide = torch.zeros((nslice, nrow, ncol + 3), dtype=dtype, device=cuda)
@@ -78,7 +94,7 @@ def test_non_finite_samples_reach_only_their_pixels(cuda, bad):
     ang = np.linspace(0.0, np.pi, nrow)
     t = torch.from_numpy(x).to(cuda)
     got = R.backproject(t, ang, 31.2)
-    ref = R.backproject(t, ang, 31.2, staging="cp.async")
+    ref = _gather(t, ang, 31.2)
     assert torch.equal(got.isnan(), ref.isnan())
     assert torch.equal(got.isinf(), ref.isinf())
     assert bool(got[:, 4].isfinite().all()) and not bool(
@@ -99,3 +115,40 @@ def test_same_bits_twice_and_under_capture(cuda):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(a, out)
+
+
+@pytest.mark.parametrize("edge_pad", [False, True])
+@pytest.mark.parametrize("nrow,nslice,ncol", [
+    (64, 1, 33), (65, 1, 100), (200, 1, 64), (97, 2, 65), (70, 3, 130),
+    (131, 4, 40), (181, 7, 96), (300, 14, 50)])
+def test_angle_groups_against_oracle(cuda, nrow, nslice, ncol, edge_pad):
+    """Few tiles: the angles are split over CTAs, the groups' compensated
+    totals are added in FP64 and rounded once (positions carry the gather
+    kernel's 1e-5 bins, as without groups)."""
+    assert nat.call("atb_backproject_stack_workspace", nat.F32, nrow, nslice,
+                    ncol) > 0
+    ang = np.linspace(0.0, np.pi, nrow)
+    x = _stack(nrow, nslice, ncol, nrow)
+    got = _check(x, ang, ncol / 2 - 1.3, edge_pad, cuda)
+    one = _gather(torch.from_numpy(x).to(cuda), ang, ncol / 2 - 1.3,
+                  edge_pad).cpu().numpy()
+    assert O.rel_l2(got, one) < 3e-7
+
+
+def test_tiles_outside_the_mask_are_zero(cuda):
+    nrow, ncol = 90, 200
+    ang = np.linspace(0.0, np.pi, nrow)
+    d = np.arange(ncol) - ncol // 2
+    for nslice in (1, 2, 5):
+        x = _stack(nrow, nslice, ncol)
+        t = torch.from_numpy(x).to(cuda)
+        for r in (3.0, 60.0, 100.0):
+            keep = d[None] ** 2 + d[:, None] ** 2 <= r * r
+            for staging in ("tma", "cp.async"):
+                out = torch.full((ncol, nslice, ncol), np.nan, device=cuda)
+                R.backproject(t, ang, 99.0, mask_r2=r * r, out=out,
+                              staging=staging)
+                got = out.cpu().numpy()
+                ref = O.back_projection(x[:, 0], ang, 99.0, False) * keep
+                assert O.rel_l2(got[:, 0], ref) < TOL
+                assert not np.any(got[:, nslice - 1][~keep])
