@@ -16,6 +16,8 @@ EXPORTS = ("atb_version", "atb_last_error", "atb_copy_2d", "atb_filter_length", 
            "atb_filter_rows", "atb_neg_log", "atb_backproject",
            "atb_backproject_status", "atb_backproject_centers",
            "atb_backproject_stack_workspace", "atb_backproject_stack",
+           "atb_backproject_centers_workspace",
+           "atb_backproject_centers_stack",
            "atb_radon_workspace", "atb_radon_adjoint", "atb_bp_batch_plan",
            "atb_backproject_batch", "atb_backproject_batch_noalloc",
            "atb_gaussian_rows",
@@ -96,6 +98,12 @@ _SIGS = {
         _vp, _c_i64, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_double,
         ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_double,
         ctypes.c_float, _vp, _c_i64, _c_i64, ctypes.c_int, _vp]),
+    "atb_backproject_centers_workspace": (_c_i64, [
+        ctypes.c_int, ctypes.c_int, ctypes.c_int]),
+    "atb_backproject_centers_stack": (ctypes.c_int, [
+        _vp, _c_i64, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_double,
+        ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_double,
+        ctypes.c_float, _vp, _c_i64, _c_i64, ctypes.c_int, _vp, _c_i64, _vp]),
     "atb_radon_workspace": (_c_i64, [ctypes.c_int, ctypes.c_int]),
     "atb_radon_adjoint": (ctypes.c_int, [
         _vp, _c_i64, _c_i64, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp,

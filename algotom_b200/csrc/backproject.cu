@@ -125,6 +125,7 @@ struct BPArgs {
   // [ngroup][nslice][ncol][ncol] (total, compensation)
   int ngroup, group_rows;
   int row0;  // first angle of this CTA's group
+  double interior;  // >= 0: leave the blocks of bp_interior to another kernel
   float2 *part;
 };
 
@@ -877,7 +878,11 @@ __global__ void __launch_bounds__(BPCfg<T, S, V>::kThreads, BPCfg<T, S, V>::kMin
     bp_kernel(BPArgs a, const __grid_constant__ CUtensorMap tmap) {
   using K = BPCfg<T, S, V>;
   extern __shared__ __align__(16) unsigned char smem[];
-  if (a.gate && !__syncthreads_or((int)threadIdx.x < a.ngate && a.gate[threadIdx.x] >= 0x7f800000u)) return;
+  if (a.gate) {
+    const bool finite = !__syncthreads_or((int)threadIdx.x < a.ngate && a.gate[threadIdx.x] >= 0x7f800000u);
+    if (finite && (a.interior < 0.0 || atb::bp_interior(blockIdx.x * K::TX, blockIdx.y * K::TY, a.ncol, a.interior)))
+      return;
+  }
   int bz = blockIdx.z;
   if (a.part) {  // this CTA's angle group
     const int nz = gridDim.z / a.ngroup, g = bz / nz;
@@ -934,6 +939,7 @@ __global__ void __launch_bounds__(BPCfg<T, 1, V>::kThreads, BPCfg<T, 1, V>::kMin
     a.spacing = 0;
     a.gate = nullptr;
     a.ngate = 0;
+    a.interior = -1.0;
     a.ngroup = 1;
     a.row0 = 0;
     a.part = nullptr;
@@ -1155,6 +1161,7 @@ int atb::bp_gather(const void *sino, int sino_dtype, int64_t sino_row_stride, in
   a.spacing = 0;
   a.gate = gate;
   a.ngate = nslice;
+  a.interior = -1.0;
   {
     const int ve = sino_dtype == ATB_F32 ? 4 : 8;  // elements per 16-byte vector
     a.vec16 = (reinterpret_cast<uintptr_t>(sino) % 16) == 0 && sino_row_stride % ve == 0 &&
@@ -1204,6 +1211,14 @@ extern "C" int atb_backproject_centers(const float *sino, int64_t sino_row_strid
                                        const double *trig, double center, int spacing, int ncenter, int edge_pad,
                                        double mask_r2, float scale, float *out, int64_t out_row_stride,
                                        int64_t out_center_stride, int flags, void *stream) {
+  return atb::bp_gather_centers(sino, sino_row_stride, nrow, ncol, trig, center, spacing, ncenter, edge_pad, mask_r2,
+                                scale, out, out_row_stride, out_center_stride, flags, nullptr, 0, -1.0, stream);
+}
+
+int atb::bp_gather_centers(const float *sino, int64_t sino_row_stride, int nrow, int ncol, const double *trig,
+                           double center, int spacing, int ncenter, int edge_pad, double mask_r2, float scale,
+                           float *out, int64_t out_row_stride, int64_t out_center_stride, int flags,
+                           const unsigned *gate, int ngate, double interior, void *stream) {
   if (!sino || !trig || !out) return atb::fail(ATB_EINVAL, "atb_backproject_centers: null pointer");
   if (nrow < 1 || ncol < 1 || ncenter < 1)
     return atb::fail(ATB_EINVAL, "atb_backproject_centers: bad shape nrow=%d ncol=%d ncenter=%d", nrow, ncol,
@@ -1232,14 +1247,17 @@ extern "C" int atb_backproject_centers(const float *sino, int64_t sino_row_strid
   a.inject = 0;
   a.wait_polls = kWaitPolls;
   a.spacing = spacing;
-  a.gate = nullptr;
-  a.ngate = 0;
+  a.gate = gate;
+  a.ngate = ngate;
+  a.interior = interior;
   a.ngroup = 1;
   a.row0 = 0;
   a.part = nullptr;
   a.vec16 = (reinterpret_cast<uintptr_t>(sino) % 16) == 0 && sino_row_stride % 4 == 0 && ncol % 4 == 0;
   cudaStream_t st = atb::as_stream(stream);
-  // four centres per CTA, then the remainder
+  // four centres per CTA, then the remainder (where only some blocks are done,
+  // all in tiles of one shape)
+  if (interior >= 0.0) return launch_bp<float, 4, false, 0, true>(a, ncenter, st);
   const int n4 = (ncenter / 4) * 4;
   int rc = ATB_OK;
   if (n4 > 0) rc = launch_bp<float, 4, false, 0, true>(a, n4, st);

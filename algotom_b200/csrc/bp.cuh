@@ -16,6 +16,14 @@ int bp_gather(const void *sino, int sino_dtype, int64_t sino_row_stride, int64_t
               void *work, void *stream);
 long long bp_gather_workspace(int nrow, int nslice, int ncol);  // 0: none is used
 
+// atb_backproject_centers (same arguments); with interior >= 0 only the blocks
+// of pixels that bp_interior does not hold for, unless the gate (ngate words,
+// as above) shows a sample that is not finite.
+int bp_gather_centers(const float *sino, int64_t sino_row_stride, int nrow, int ncol, const double *trig,
+                      double center, int spacing, int ncenter, int edge_pad, double mask_r2, float scale, float *out,
+                      int64_t out_row_stride, int64_t out_center_stride, int flags, const unsigned *gate, int ngate,
+                      double interior, void *stream);
+
 // Status word of the tensor-core back-projector, as atb_backproject_status.
 int bp_mma_status(int reset);
 
@@ -25,6 +33,18 @@ int bp_mma_status(int reset);
 __host__ __device__ inline int bp_sample_exponent(unsigned maxbits) {
   const int e = 14 - ((int)(maxbits >> 23) - 127);
   return e < -126 ? -126 : (e > 126 ? 126 : e);
+}
+
+// Whether every pixel of the 64 x 32 block (the gather kernel's tile of four
+// slices) around pixel (x, y) lies within
+// `radius` of the image centre, so that no position of it leaves a detector
+// that reaches `radius` to both sides of the rotation axis.
+__device__ __forceinline__ bool bp_interior(int x, int y, int ncol, double radius) {
+  const double ic = 0.5 * (double)(ncol - 1);
+  const int bx = x & ~63, by = y & ~31;
+  const double dx = fmax(fabs((double)bx - ic), fabs((double)min(bx + 63, ncol - 1) - ic));
+  const double dy = fmax(fabs((double)by - ic), fabs((double)min(by + 31, ncol - 1) - ic));
+  return radius > 0.0 && dx * dx + dy * dy <= radius * radius;
 }
 #endif
 

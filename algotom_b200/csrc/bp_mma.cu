@@ -81,11 +81,11 @@ constexpr int kStep = 4;                  // angles per weight slot
 // 10.6, 10.1 and 10.0 ms.
 constexpr int kFoldPlain = 4, kFoldEdge = 2;
 // warps 0-15 form the weights (four for each tile), 16-19 keep the totals,
-// 20-23 issue a tile's MMAs each, 24-27 stage (every fourth chunk each: one
-// warp alone, waiting for its FP64 results, was slower than the rest)
+// 20-23 issue a tile's MMAs each, 25-27 stage (every third chunk each: one warp
+// alone, waiting for its FP64 results, takes 2.29 ms at 361 x 1024 with 32
+// slices where three take 1.81; four, with warp 24, 1.86)
 constexpr int kTotals = 16, kIssuers = 20, kProducers = 24;
 constexpr int kThreads = 28 * 32;
-static_assert(kRing == 4, "a staging warp for each slot of the ring");
 // registers per thread of the three kinds: 512 x 64 + 128 x 168 + 256 x 40 =
 // 896 x 72, what the block is launched with
 constexpr int kRegsWeights = 64, kRegsTotals = 168, kRegsHelpers = 40;
@@ -107,6 +107,7 @@ struct MmaArgs {
   float scale;
   float *out;
   long long ors, oss;
+  double interior;  // >= 0: only the blocks of bp_interior (centre groups)
 };
 
 // parameters of one (angle, tile)
@@ -353,6 +354,7 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
   const int ncol = a.ncol, cm = ncol / 2;
   // non-finite samples: the gather kernel takes the stack
   if (__syncthreads_or(tid < S && a.maxbits[tid] >= kInfBits)) return;
+  if (a.interior >= 0.0 && !atb::bp_interior(x0, y0, ncol, a.interior)) return;
   // a region wholly outside the circle mask is zero
   if (a.mask_r2 >= 0.0) {
     const long long dx = max(0, max(x0 - cm, cm - (x0 + kRegion - 1)));
@@ -405,8 +407,8 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
   if (warp >= kProducers) {
     // lane = angle of the chunk and tile
     const int ai = lane >> 2;
-    const int r = warp - kProducers;
-    for (int k = r; k < nchunk; k += kRing) {
+    for (int k = warp - kProducers - 1; warp > kProducers && k < nchunk; k += 3) {
+      const int r = k % kRing;
       if (k >= kRing) mbar_wait(&empty[r], (unsigned)((k / kRing - 1) & 1), bad);
       unsigned char *dst = smem + (size_t)(r * kChunk + ai) * K::kAngleBytes;
       const int e = r * kChunk * 4 + lane;
@@ -651,6 +653,38 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
   }
 }
 
+// The S "slices" of a centre group: slice m is the one row of each angle, read m
+// spacing bins further on.  One word of maxbits serves them all (the others
+// repeat it).
+__global__ void __launch_bounds__(256) pack_centers_kernel(const float *sino, long long srs, int ncol, int nsl, int S,
+                                                           int spacing, unsigned *maxbits, uint4 *dst) {
+  const int i = blockIdx.y, g = blockIdx.z;
+  const unsigned bits = maxbits[0];
+  if (i == 0 && blockIdx.x == 0 && threadIdx.x < 8) maxbits[S + 8 * g + threadIdx.x] = bits;
+  const float sc = __int_as_float((atb::bp_sample_exponent(bits) + 127) << 23);
+  const float *row = sino + i * srs;
+  uint4 *hi = dst + ((long long)i * (S / 4) + g) * ncol, *lo = hi + (long long)(S / 8) * ncol;
+  for (int d = blockIdx.x * 256 + threadIdx.x; d < ncol; d += gridDim.x * 256) {
+    unsigned h[4], l[4];
+#pragma unroll
+    for (int u = 0; u < 8; u += 2) {
+      float v[2];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int m = 8 * g + u + t, b = d + m * spacing;
+        v[t] = m < nsl && b < ncol ? __ldg(row + b) * sc : 0.f;
+      }
+      const __half2 hh = __floats2half2_rn(v[0], v[1]);
+      const float2 hf = __half22float2(hh);
+      const __half2 ll = __floats2half2_rn(v[0] - hf.x, v[1] - hf.y);
+      h[u / 2] = *reinterpret_cast<const unsigned *>(&hh);
+      l[u / 2] = *reinterpret_cast<const unsigned *>(&ll);
+    }
+    hi[d] = make_uint4(h[0], h[1], h[2], h[3]);
+    lo[d] = make_uint4(l[0], l[1], l[2], l[3]);
+  }
+}
+
 // largest |sample| of each slice as float bits (monotonic; a NaN ranks above
 // infinity).  grid (row blocks, slices), atomics on zeroed words.
 template <typename T>
@@ -732,6 +766,16 @@ int launch_mma(const MmaArgs &a, void *packed, cudaStream_t st) {
   const int n = (a.ncol + kRegion - 1) / kRegion;
   fn<<<dim3(n, n), kThreads, K::kSmem, st>>>(a, map);
   return atb::check_launch("atb_backproject_stack");
+}
+
+int launch(const MmaArgs &a, int S, void *packed, cudaStream_t st) {
+  if (a.edge_pad)
+    return S == 16   ? launch_mma<16, kFoldEdge>(a, packed, st)
+           : S == 24 ? launch_mma<24, kFoldEdge>(a, packed, st)
+                     : launch_mma<32, kFoldEdge>(a, packed, st);
+  return S == 16   ? launch_mma<16, kFoldPlain>(a, packed, st)
+         : S == 24 ? launch_mma<24, kFoldPlain>(a, packed, st)
+                   : launch_mma<32, kFoldPlain>(a, packed, st);
 }
 
 template <typename T>
@@ -818,15 +862,8 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
       a.nrow = nrow; a.ncol = ncol; a.nsl = n;
       a.center = center; a.edge_pad = edge_pad ? 1 : 0; a.mask_r2 = mask_r2; a.scale = scale;
             a.out = dst; a.ors = out_row_stride; a.oss = out_slice_stride;
-      void *packed = static_cast<unsigned char *>(workspace) + kHeader;
-      if (edge_pad)
-        rc = S == 16   ? launch_mma<16, kFoldEdge>(a, packed, st)
-             : S == 24 ? launch_mma<24, kFoldEdge>(a, packed, st)
-                       : launch_mma<32, kFoldEdge>(a, packed, st);
-      else
-        rc = S == 16   ? launch_mma<16, kFoldPlain>(a, packed, st)
-             : S == 24 ? launch_mma<24, kFoldPlain>(a, packed, st)
-                       : launch_mma<32, kFoldPlain>(a, packed, st);
+      a.interior = -1.0;
+      rc = launch(a, S, static_cast<unsigned char *>(workspace) + kHeader, st);
       if (rc != ATB_OK) return rc;
       // runs only where a sample is not finite
       rc = atb::bp_gather(src, sino_dtype, sino_row_stride, sino_slice_stride, nrow, n, ncol, trig, center, edge_pad,
@@ -839,4 +876,61 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
                         sino_dtype, sino_row_stride, sino_slice_stride, nrow, nslice - first, ncol, trig, center,
                         edge_pad, mask_r2, scale, out ? out + (int64_t)first * out_slice_stride : out, out_row_stride,
                         out_slice_stride, flags, nullptr, work_ok ? workspace : nullptr, stream);
+}
+
+extern "C" int64_t atb_backproject_centers_workspace(int nrow, int ncol, int ncenter) {
+  if (nrow < 1 || ncol < 1 || ncenter < 1 || nrow > 65535 || ncol > (1 << 16)) return 0;
+  const int n = next_group(ATB_F32, ncenter);
+  return n ? kHeader + (int64_t)nrow * ncol * padded(n) * 4 : 0;
+}
+
+extern "C" int atb_backproject_centers_stack(const float *sino, int64_t sino_row_stride, int nrow, int ncol,
+                                             const double *trig, double center, int spacing, int ncenter,
+                                             int edge_pad, double mask_r2, float scale, float *out,
+                                             int64_t out_row_stride, int64_t out_center_stride, int flags,
+                                             void *workspace, int64_t workspace_bytes, void *stream) {
+  cudaStream_t st = atb::as_stream(stream);
+  const int64_t need = atb_backproject_centers_workspace(nrow, ncol, ncenter);
+  int first = 0;
+  // (arguments that atb_backproject_centers refuses go there)
+  if (sino && trig && out && spacing >= 1 && spacing <= 56 && center >= 0.0 &&
+      center + (double)(ncenter - 1) * (double)spacing < (double)ncol && need > 0 && workspace &&
+      workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 128 == 0) {
+    unsigned *maxbits = static_cast<unsigned *>(workspace);
+    uint4 *packed = reinterpret_cast<uint4 *>(static_cast<unsigned char *>(workspace) + kHeader);
+    if (cudaMemsetAsync(workspace, 0, kHeader, st) != cudaSuccess)
+      return atb::fail(ATB_ECUDA, "atb_backproject_centers_stack: %s", cudaGetErrorString(cudaGetLastError()));
+    absmax_kernel<float><<<dim3(nrow < 256 ? nrow : 256, 1), 256, 0, st>>>(sino, sino_row_stride, 0, nrow, ncol, maxbits);
+    int rc = atb::check_launch("atb_backproject_centers_stack (scan)");
+    if (rc != ATB_OK) return rc;
+    for (int n; (n = next_group(ATB_F32, ncenter - first)) > 0; first += n) {
+      const int S = padded(n);
+      const double c0 = center + (double)first * (double)spacing, c1 = c0 + (double)(n - 1) * (double)spacing;
+      // samples of the first centre's frame: later centres read further on
+      pack_centers_kernel<<<dim3((ncol + 255) / 256, nrow, S / 8), 256, 0, st>>>(sino, sino_row_stride, ncol, n, S,
+                                                                                spacing, maxbits, packed);
+      rc = atb::check_launch("atb_backproject_centers_stack (pack)");
+      if (rc != ATB_OK) return rc;
+      MmaArgs a;
+      a.maxbits = maxbits + S;
+      a.trig = reinterpret_cast<const double2 *>(trig);
+      a.nrow = nrow; a.ncol = ncol; a.nsl = n;
+      a.center = c0; a.edge_pad = edge_pad ? 1 : 0; a.mask_r2 = mask_r2; a.scale = scale;
+      a.out = out + (int64_t)first * out_center_stride; a.ors = out_row_stride; a.oss = out_center_stride;
+      const double reach = (c0 < (double)(ncol - 1) - c1 ? c0 : (double)(ncol - 1) - c1) - 1e-2;
+      a.interior = reach > 0.0 ? reach : 0.0;
+      rc = launch(a, S, packed, st);
+      if (rc != ATB_OK) return rc;
+      // the blocks whose positions reach an edge of the detector for some
+      // centre: each centre has its own edges there
+      rc = atb::bp_gather_centers(sino, sino_row_stride, nrow, ncol, trig, c0, spacing, n, edge_pad, mask_r2, scale,
+                                  a.out, out_row_stride, out_center_stride, flags, maxbits, 1, a.interior, stream);
+      if (rc != ATB_OK) return rc;
+    }
+    if (first == ncenter) return ATB_OK;
+  }
+  return atb::bp_gather_centers(sino, sino_row_stride, nrow, ncol, trig, center + (double)first * (double)spacing,
+                                spacing, ncenter - first, edge_pad, mask_r2, scale,
+                                out ? out + (int64_t)first * out_center_stride : out, out_row_stride,
+                                out_center_stride, flags, nullptr, 0, -1.0, stream);
 }

@@ -21,6 +21,7 @@ come back to the host; a custom ``metric_function`` gets each
 reconstruction as a NumPy array, as in the reference.
 """
 import ctypes
+import functools
 
 import numpy as np
 import torch
@@ -136,6 +137,14 @@ def _backproject_items(items, device, variant):
     return items_dev, units_dev, counter
 
 
+@functools.lru_cache(maxsize=256)
+def _centers_need(nrow, ncol, count):
+    """Scratch bytes of ``atb_backproject_centers_stack``; 0 where it is
+    ``atb_backproject_centers`` (groups below 15)."""
+    return 0 if count < 15 else nat.call("atb_backproject_centers_workspace",
+                                         nrow, ncol, count)
+
+
 def _centre_groups(centers, max_classes=16, max_spacing=56):
     """Split candidate centres into progressions whose float32 values differ
     by whole pixels: ``[(r, R, c0, spacing, count)]`` where candidates
@@ -212,15 +221,21 @@ class _Source:
                  for c in centers}
         groups = _centre_groups(centers) if len(masks) == 1 else None
         if groups is not None:
-            # candidates a whole number of pixels apart: 4 per CTA
+            # candidates a whole number of pixels apart share positions
             mask_r2 = masks.pop()
             st = R._stream_ptr(dev)
+            need = max(_centers_need(nrow, ncol, grp[4]) for grp in groups)
+            ws = R._stack_workspace(need, dev) if need > 0 else None
             for r, ncls, c0, g, cnt in groups:
-                nat.call("atb_backproject_centers", self.src.data_ptr(),
-                         self.src_rs, nrow, ncol, self.trig.data_ptr(), c0,
-                         g, cnt, 0 if fbp else 1, mask_r2,
-                         scale if fbp else 1.0, out[r].data_ptr(),
-                         out.stride(1), ncls * out.stride(0), 0, st)
+                args = (self.src.data_ptr(), self.src_rs, nrow, ncol,
+                        self.trig.data_ptr(), c0, g, cnt, 0 if fbp else 1,
+                        mask_r2, scale if fbp else 1.0, out[r].data_ptr(),
+                        out.stride(1), ncls * out.stride(0), 0)
+                if ws is not None:
+                    nat.call("atb_backproject_centers_stack", *args,
+                             ws.data_ptr(), need, st)
+                else:
+                    nat.call("atb_backproject_centers", *args, st)
         items = []
         for k, c in enumerate([] if groups is not None else centers):
             it = nat.BpItem()

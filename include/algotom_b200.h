@@ -269,6 +269,26 @@ int atb_backproject_centers(const float *sino, int64_t sino_row_stride,
                             void *stream);
 
 /*
+ * atb_backproject_centers, given a workspace: groups of 15 and more centres run
+ * on the tensor cores (up to 32 per launch) where no position leaves the
+ * detector for any of them, the rest of the image and every call without a
+ * (large enough) workspace as atb_backproject_centers does.  Results differ by
+ * rounding only.
+ *
+ *   workspace  128-byte aligned device scratch of
+ *              atb_backproject_centers_workspace bytes (0: none is used)
+ */
+int64_t atb_backproject_centers_workspace(int nrow, int ncol, int ncenter);
+int atb_backproject_centers_stack(const float *sino, int64_t sino_row_stride,
+                                  int nrow, int ncol, const double *trig,
+                                  double center, int spacing, int ncenter,
+                                  int edge_pad, double mask_r2, float scale,
+                                  float *out, int64_t out_row_stride,
+                                  int64_t out_center_stride, int flags,
+                                  void *workspace, int64_t workspace_bytes,
+                                  void *stream);
+
+/*
  * Status word of the back-projection kernels: bit 0 is set when a CTA gave
  * up waiting (after about 70 ms) for a TMA window load and left its tile
  * unwritten.  Returns the word (0 = no such event since the last reset) and

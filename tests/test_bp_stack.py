@@ -152,3 +152,28 @@ def test_tiles_outside_the_mask_are_zero(cuda):
                 ref = O.back_projection(x[:, 0], ang, 99.0, False) * keep
                 assert O.rel_l2(got[:, 0], ref) < TOL
                 assert not np.any(got[:, nslice - 1][~keep])
+
+
+@pytest.mark.parametrize("edge_pad", [0, 1])
+@pytest.mark.parametrize("n,spacing,c0", [(15, 1, 140.25), (24, 2, 130.0),
+                                          (33, 1, 150.5), (47, 3, 20.75),
+                                          (20, 9, 1.0)])
+def test_centre_groups_against_oracle(cuda, n, spacing, c0, edge_pad):
+    """Groups of candidate centres: blocks inside every centre's detector on
+    the tensor cores, the others on the gather kernel."""
+    nrow, ncol = 41, 301
+    ang = np.linspace(0.0, np.pi, nrow)
+    x = _stack(nrow, 1, ncol)
+    t = torch.from_numpy(x[:, 0]).to(cuda)
+    need = nat.call("atb_backproject_centers_workspace", nrow, ncol, n)
+    assert need > 0
+    ws = torch.empty(need, dtype=torch.uint8, device=cuda)
+    out = torch.full((n, ncol, ncol), np.nan, device=cuda)
+    nat.call("atb_backproject_centers_stack", t.data_ptr(), t.stride(0), nrow,
+             ncol, R._trig(ang, cuda).data_ptr(), c0, spacing, n, edge_pad,
+             -1.0, 1.0, out.data_ptr(), out.stride(1), out.stride(0), 0,
+             ws.data_ptr(), need, R._stream_ptr(cuda))
+    got = out.cpu().numpy()
+    for m in (0, n // 2, n - 1):
+        ref = O.back_projection(x[:, 0], ang, c0 + m * spacing, edge_pad)
+        assert O.rel_l2(got[m], ref) < TOL, m
