@@ -497,7 +497,7 @@ int transform_length(int ncol, int pad) {
   return -1;
 }
 
-// radices of t, 8s and 4s first, then the odd ones, then a last 2
+// radices of t: the odd ones, 8s, 4s, a last 2
 bool make_plan(int t, const double2 *tw, Plan &pl) {
   pl.n = t;
   pl.tw = tw;
@@ -509,14 +509,16 @@ bool make_plan(int t, const double2 *tw, Plan &pl) {
     r /= p;
     return true;
   };
-  while (r % 8 == 0)
-    if (!push(8)) return false;
-  while (r % 4 == 0)
-    if (!push(4)) return false;
+  // odd radices first: the first stage writes with its radix as the stride
+  // between threads, which conflicts in the banks for an even one
   static const int odd[] = {13, 11, 7, 5, 3};
   for (int p : odd)
     while (r % p == 0)
       if (!push(p)) return false;
+  while (r % 8 == 0)
+    if (!push(8)) return false;
+  while (r % 4 == 0)
+    if (!push(4)) return false;
   while (r % 2 == 0)
     if (!push(2)) return false;
   if (r != 1) return false;

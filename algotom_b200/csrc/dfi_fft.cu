@@ -41,6 +41,7 @@ namespace {
 
 using atb::fft::cmul;
 using atb::fft::cmulc;
+using atb::fft::ip_at;
 using atb::fft::IpPlan;
 
 constexpr int kThreads = 512;
@@ -59,23 +60,31 @@ struct Tables {
 template <bool INV>
 __device__ void bluestein(double2 *x, int w, const IpPlan &pl, const double2 *tws, const Tables &t) {
   const int M = pl.n;
+  // into the transform's order: elements move within aligned groups of eight,
+  // which lie in one warp's hands
   for (int n = threadIdx.x; n < M; n += blockDim.x) {
+    double2 v = make_double2(0.0, 0.0);
     if (n < w) {
       const double2 b = __ldg(t.chirp + n);
-      x[n] = INV ? cmul(x[n], b) : cmulc(x[n], b);
-    } else {
-      x[n] = make_double2(0.0, 0.0);
+      v = INV ? cmul(x[n], b) : cmulc(x[n], b);
     }
+    __syncwarp(__activemask());
+    x[ip_at(n)] = v;
   }
   __syncthreads();
   atb::fft::ip_run<false>(x, pl, tws);
   const double2 *B = INV ? t.binv : t.bfwd;
-  for (int p = threadIdx.x; p < M; p += blockDim.x) x[p] = cmul(x[p], __ldg(B + p));
+  for (int p = threadIdx.x; p < M; p += blockDim.x) x[ip_at(p)] = cmul(x[ip_at(p)], __ldg(B + p));
   __syncthreads();
   atb::fft::ip_run<true>(x, pl, tws);
-  for (int k = threadIdx.x; k < w; k += blockDim.x) {
-    const double2 b = __ldg(t.chirp + k);
-    x[k] = INV ? cmul(x[k], b) : cmulc(x[k], b);
+  for (int k = threadIdx.x; k < M; k += blockDim.x) {  // (whole groups of eight)
+    double2 v = x[ip_at(k)];
+    if (k < w) {
+      const double2 b = __ldg(t.chirp + k);
+      v = INV ? cmul(v, b) : cmulc(v, b);
+    }
+    __syncwarp(__activemask());
+    x[k] = v;
   }
   __syncthreads();
 }
@@ -95,13 +104,13 @@ __global__ void __launch_bounds__(kThreads) chirp_setup_kernel(int w, const __gr
     if (m < w) v = __ldg(t.chirp + m);
     else if (M - m < w) v = __ldg(t.chirp + (M - m));
     if (conj) v.y = -v.y;
-    sm[m] = v;
+    sm[ip_at(m)] = v;
   }
   __syncthreads();
   atb::fft::ip_run<false>(sm, pl, tws);
   double2 *out = conj ? binv : bfwd;
   const double s = 1.0 / (double)M;
-  for (int p = threadIdx.x; p < M; p += blockDim.x) out[p] = make_double2(sm[p].x * s, sm[p].y * s);
+  for (int p = threadIdx.x; p < M; p += blockDim.x) out[p] = make_double2(sm[ip_at(p)].x * s, sm[ip_at(p)].y * s);
 }
 
 // ---- padding (np.pad(row, pad, mode), numpy's ten modes, float32)
@@ -394,6 +403,11 @@ bool plan_for(int w, IpPlan &pl, int &M) {
 
 size_t smem_bytes(int M) { return ((size_t)M + (size_t)atb::fft::twiddle_entries(M)) * sizeof(double2); }
 
+// Threads of a CTA: 512 at 128 registers fill an SM's register file, so the
+// shorter transforms, whose buffers leave room for more CTAs, take fewer threads:
+// one CTA's barriers are then covered by another's work.
+int cta_threads(int M) { return M >= 8192 ? 512 : M >= 4096 ? 256 : 128; }
+
 int prepare(int w, const char *what, IpPlan &pl, int &M) {
   if (w < 2) return atb::fail(ATB_EINVAL, "%s: width %d", what, w);
   if (!plan_for(w, pl, M))
@@ -429,7 +443,7 @@ extern "C" int atb_dfi_fft_setup(int w, const void *chirp, const void *twiddle, 
   int M = 0;
   const int rc = prepare(w, "atb_dfi_fft_setup", pl, M);
   if (rc != ATB_OK) return rc;
-  chirp_setup_kernel<<<2, kThreads, smem_bytes(M), atb::as_stream(stream)>>>(
+  chirp_setup_kernel<<<2, cta_threads(M), smem_bytes(M), atb::as_stream(stream)>>>(
       w, pl, tables(chirp, twiddle, nullptr, nullptr), static_cast<double2 *>(bfwd), static_cast<double2 *>(binv));
   return atb::check_launch("atb_dfi_fft_setup");
 }
@@ -458,7 +472,7 @@ extern "C" int atb_dfi_rows(const float *src, int64_t src_row_stride, int64_t sr
   a.window = window; a.nonpositive = nonpositive;
   a.dst = static_cast<double2 *>(dst); a.drs = dst_row_stride; a.dss = dst_slice_stride;
   const dim3 grid((nrow + 1) / 2, nslice);
-  dfi_rows_kernel<<<grid, kThreads, smem_bytes(M), st>>>(a, pl, tables(chirp, twiddle, bfwd, binv));
+  dfi_rows_kernel<<<grid, cta_threads(M), smem_bytes(M), st>>>(a, pl, tables(chirp, twiddle, bfwd, binv));
   return atb::check_launch("atb_dfi_rows");
 }
 
@@ -493,9 +507,9 @@ extern "C" int atb_dfi_inverse(const void *coef, int64_t coef_row_stride, int64_
   a.out = out; a.ors = out_row_stride; a.oss = out_slice_stride; a.out_f32 = out_f32 ? 1 : 0;
   const Tables t = tables(chirp, twiddle, bfwd, binv);
   cudaStream_t st = atb::as_stream(stream);
-  dfi_inv_rows_kernel<<<dim3(w / 2 + 1, nslice), kThreads, smem_bytes(M), st>>>(a, pl, t);
+  dfi_inv_rows_kernel<<<dim3(w / 2 + 1, nslice), cta_threads(M), smem_bytes(M), st>>>(a, pl, t);
   const int r = atb::check_launch("atb_dfi_inverse (rows)");
   if (r != ATB_OK) return r;
-  dfi_inv_cols_kernel<<<dim3((ncol + 1) / 2, nslice), kThreads, smem_bytes(M), st>>>(a, pl, t);
+  dfi_inv_cols_kernel<<<dim3((ncol + 1) / 2, nslice), cta_threads(M), smem_bytes(M), st>>>(a, pl, t);
   return atb::check_launch("atb_dfi_inverse (columns)");
 }

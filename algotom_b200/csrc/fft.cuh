@@ -159,16 +159,22 @@ __device__ __forceinline__ void stage(const double2 *__restrict__ in, double2 *_
 #pragma unroll
     for (int t = 0; t < (P - 1) / 2; ++t) rc[t] = pl.rc[odd_slot(P)][t];
   }
+  // j / L by a multiplication (exact for j, L < 2^14)
+  const unsigned magic = L > 1 ? 0xffffffffu / (unsigned)L + 1u : 0u;
   for (int j = threadIdx.x; j < m; j += blockDim.x) {
-    const int i = j / L, k = j - i * L;
+    const int i = L > 1 ? (int)__umulhi((unsigned)j, magic) : j, k = j - i * L;
     double2 v[P];
 #pragma unroll
     for (int r = 0; r < P; ++r) v[r] = in[j + r * m];
     if (k > 0) {
+      // one table value and its powers: P - 1 look-ups of two values each
+      // were two thirds of the stage's shared-memory traffic
+      const double2 w = twiddle(tws, k * tstep);
+      double2 wr = w;
 #pragma unroll
       for (int r = 1; r < P; ++r) {
-        const double2 w = twiddle(tws, r * k * tstep);
-        v[r] = INV ? cmulc(v[r], w) : cmul(v[r], w);
+        v[r] = INV ? cmulc(v[r], wr) : cmul(v[r], wr);
+        if (r + 1 < P) wr = cmul(wr, w);
       }
     }
     dft<P, INV>(v, rc);
@@ -269,6 +275,12 @@ __device__ __forceinline__ void ip_butterfly(double2 (&v)[R], int n1, int tstep,
   if constexpr (INV) dft<R, true>(v, rc);
 }
 
+// Where element i of the buffer sits: the stages' butterflies meet elements 8
+// apart (the last forward stage) in one instruction, which share banks in
+// natural order (8 ways); with the low three bits exchanged by the next three
+// neither these nor consecutive elements do.
+__device__ __forceinline__ int ip_at(int i) { return i ^ ((i >> 3) & 7); }
+
 template <int R, bool INV>
 __device__ __forceinline__ void ip_stage(double2 *x, int n, int L, const double2 *tws) {
   const int s = L / R, tstep = n / L, nq = n / R, nt = blockDim.x;
@@ -277,26 +289,25 @@ __device__ __forceinline__ void ip_stage(double2 *x, int n, int L, const double2
     const int q1 = q0 + nt;
     const bool two = q1 < nq;
     const int n10 = q0 & (s - 1), n11 = q1 & (s - 1);
-    double2 *p0 = x + (q0 >> sh) * L + n10;
-    double2 *p1 = x + (q1 >> sh) * L + n11;
+    const int p0 = (q0 >> sh) * L + n10, p1 = (q1 >> sh) * L + n11;
     double2 v0[R], v1[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      v0[j] = p0[j * s];
-      v1[j] = two ? p1[j * s] : make_double2(0.0, 0.0);
+      v0[j] = x[ip_at(p0 + j * s)];
+      v1[j] = two ? x[ip_at(p1 + j * s)] : make_double2(0.0, 0.0);
     }
     ip_butterfly<R, INV>(v0, n10, tstep, tws);
     ip_butterfly<R, INV>(v1, n11, tstep, tws);
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      p0[j * s] = v0[j];
-      if (two) p1[j * s] = v1[j];
+      x[ip_at(p0 + j * s)] = v0[j];
+      if (two) x[ip_at(p1 + j * s)] = v1[j];
     }
   }
 }
 
-// every thread of the CTA calls these; a barrier separates the stages and
-// follows the last one
+// Every thread of the CTA calls these; a barrier separates the stages and
+// follows the last one.  Element i is x[ip_at(i)] before and after.
 template <bool INV>
 __device__ void ip_run(double2 *x, const IpPlan &pl, const double2 *tws) {
   if constexpr (!INV) {
