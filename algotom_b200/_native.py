@@ -24,7 +24,8 @@ EXPORTS = ("atb_version", "atb_last_error", "atb_copy_2d", "atb_filter_length", 
            "atb_gaussian_cols", "atb_zoom_linear", "atb_image_range",
            "atb_slice_metric_workspace", "atb_slice_metric",
            "atb_slice_entropy64", "atb_vertical_backproject",
-           "atb_vertical_workspace", "atb_flat_log", "atb_shift_rows",
+           "atb_vertical_workspace", "atb_flat_log",
+           "atb_flat_log_chunks", "atb_shift_rows",
            "atb_extend_rows", "atb_spline_prefilter", "atb_dfi_regrid",
            "atb_bpf_filter2d_length", "atb_bpf_filter2d_workspace",
            "atb_bpf_filter2d", "atb_filter_rows_batch", "atb_shift_rows_ext",
@@ -201,6 +202,10 @@ _SIGS = {
         _vp, ctypes.c_int, _c_i64, _c_i64, ctypes.c_int, ctypes.c_int,
         ctypes.c_int, _vp, _vp, _c_i64, ctypes.c_int, _vp, _c_i64, _c_i64,
         _vp, _vp]),
+    "atb_flat_log_chunks": (ctypes.c_int, [
+        _vp, ctypes.c_int, _c_i64, _c_i64, ctypes.c_int, ctypes.c_int,
+        ctypes.c_int, ctypes.c_int, _vp, _vp, _c_i64, ctypes.c_int, _vp,
+        _c_i64, _c_i64, _vp, _vp]),
 }
 
 _lib = None

@@ -209,22 +209,30 @@ int vbp_groups(int nproj, long long base) {
   return (int)(g < 1 ? 1 : g);
 }
 
+// four neighbouring samples
+__device__ __forceinline__ float4 load4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ float4 load4(const unsigned short *p) {
+  const ushort4 v = *reinterpret_cast<const ushort4 *>(p);
+  return make_float4((float)v.x, (float)v.y, (float)v.z, (float)v.w);
+}
+
 // dst = -log((src - dark) / flat_dark) with the reference's <= 0 -> 1
-// replacement; counts the replaced values in *nonpos
-template <typename T>
-__global__ void flat_log_kernel(const T *__restrict__ src, long long sps, long long srs, int nproj, int height,
-                                int width, const float *__restrict__ dark, const float *__restrict__ flat_dark,
-                                long long frs, int apply_log, float *__restrict__ dst, long long dps, long long drs,
-                                unsigned *nonpos) {
-  const long long total = (long long)nproj * height * width;
-  unsigned bad = 0;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(e % width);
-    const long long t = e / width;
-    const int i = (int)(t % height), n = (int)(t / height);
-    float v = atb::to_float(src[n * sps + i * srs + c]);
-    if (flat_dark) v = __fdiv_rn(__fsub_rn(v, dark[i * frs + c]), flat_dark[i * frs + c]);
+// replacement; counts the replaced values of each `chunk` projections in
+// nonpos[n / chunk].  A warp per row, so that the row's place is worked out once
+// (three 64-bit divisions per sample held the kernel to 1.3 TB/s); VEC: four
+// samples at a time, for rows aligned and a multiple of four long.  Memory
+// bound: 443 MB in and out in one launch, 725 us in 31 launches before.
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256) flat_log_kernel(const T *__restrict__ src, long long sps, long long srs,
+                                                       int nproj, int height, int width, int chunk,
+                                                       const float *__restrict__ dark,
+                                                       const float *__restrict__ flat_dark, long long frs,
+                                                       int apply_log, float *__restrict__ dst, long long dps,
+                                                       long long drs, unsigned *nonpos) {
+  const int lane = threadIdx.x & 31;
+  const long long rows = (long long)nproj * height;
+  auto value = [&](float v, long long f, unsigned &bad) -> float {
+    if (flat_dark) v = __fdiv_rn(__fsub_rn(v, dark[f]), flat_dark[f]);
     if (apply_log) {
       if (v <= 0.0f) {
         ++bad;
@@ -232,10 +240,46 @@ __global__ void flat_log_kernel(const T *__restrict__ src, long long sps, long l
       }
       v = -logf(v);
     }
-    dst[n * dps + i * drs + c] = v;
+    return v;
+  };
+  for (long long r = blockIdx.x * 8ll + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8ll) {
+    const int n = (int)(r / height), i = (int)(r - (long long)n * height);
+    const T *s = src + n * sps + i * srs;
+    float *d = dst + n * dps + i * drs;
+    unsigned bad = 0;
+    if constexpr (VEC) {
+#pragma unroll 2
+      for (int c = 4 * lane; c < width; c += 128) {
+        float4 v = load4(s + c);
+        v.x = value(v.x, i * frs + c, bad);
+        v.y = value(v.y, i * frs + c + 1, bad);
+        v.z = value(v.z, i * frs + c + 2, bad);
+        v.w = value(v.w, i * frs + c + 3, bad);
+        *reinterpret_cast<float4 *>(d + c) = v;
+      }
+    } else {
+      for (int c = lane; c < width; c += 32) d[c] = value(atb::to_float(s[c]), i * frs + c, bad);
+    }
+    bad = __reduce_add_sync(0xffffffffu, bad);
+    if (lane == 0 && bad) atomicAdd(nonpos + n / chunk, bad);
   }
-  for (int o = 16; o > 0; o >>= 1) bad += __shfl_xor_sync(0xffffffffu, bad, o);
-  if ((threadIdx.x & 31) == 0 && bad) atomicAdd(nonpos, bad);
+}
+
+template <typename T>
+void launch_flat_log(const void *src, long long sps, long long srs, int nproj, int height, int width, int chunk,
+                     const float *dark, const float *flat_dark, long long frs, int apply_log, float *dst,
+                     long long dps, long long drs, unsigned *nonpos, cudaStream_t st) {
+  const T *s = static_cast<const T *>(src);
+  const long long rows = (long long)nproj * height;
+  const long long blocks = (rows + 7) / 8 < 148LL * 32 ? (rows + 7) / 8 : 148LL * 32;
+  const bool vec = width % 4 == 0 && sps % 4 == 0 && srs % 4 == 0 && dps % 4 == 0 && drs % 4 == 0 &&
+                   reinterpret_cast<uintptr_t>(s) % (4 * sizeof(T)) == 0 && reinterpret_cast<uintptr_t>(dst) % 16 == 0;
+  if (vec)
+    flat_log_kernel<T, true><<<(int)blocks, 256, 0, st>>>(s, sps, srs, nproj, height, width, chunk, dark, flat_dark,
+                                                          frs, apply_log, dst, dps, drs, nonpos);
+  else
+    flat_log_kernel<T, false><<<(int)blocks, 256, 0, st>>>(s, sps, srs, nproj, height, width, chunk, dark, flat_dark,
+                                                           frs, apply_log, dst, dps, drs, nonpos);
 }
 
 }  // namespace
@@ -292,33 +336,37 @@ extern "C" int atb_vertical_backproject(const float *proj, int64_t proj_stride, 
   return atb::check_launch("atb_vertical_backproject");
 }
 
-extern "C" int atb_flat_log(const void *src, int src_dtype, int64_t src_proj_stride, int64_t src_row_stride,
-                            int nproj, int height, int width, const float *dark, const float *flat_dark,
-                            int64_t field_row_stride, int apply_log, float *dst, int64_t dst_proj_stride,
-                            int64_t dst_row_stride, unsigned *nonpos, void *stream) {
+extern "C" int atb_flat_log_chunks(const void *src, int src_dtype, int64_t src_proj_stride, int64_t src_row_stride,
+                                   int nproj, int height, int width, int chunk, const float *dark,
+                                   const float *flat_dark, int64_t field_row_stride, int apply_log, float *dst,
+                                   int64_t dst_proj_stride, int64_t dst_row_stride, unsigned *nonpos, void *stream) {
   if (!src || !dst || !nonpos) return atb::fail(ATB_EINVAL, "atb_flat_log: null pointer");
   if ((dark == nullptr) != (flat_dark == nullptr))
     return atb::fail(ATB_EINVAL, "atb_flat_log: dark and flat_dark go together");
-  if (nproj < 1 || height < 1 || width < 1)
+  if (nproj < 1 || height < 1 || width < 1 || chunk < 1)
     return atb::fail(ATB_EINVAL, "atb_flat_log: bad shape nproj=%d height=%d width=%d", nproj, height, width);
   cudaStream_t st = atb::as_stream(stream);
-  const long long total = (long long)nproj * height * width;
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148LL * 16) blocks = 148LL * 16;
   switch (src_dtype) {
     case ATB_F32:
-      flat_log_kernel<float><<<(int)blocks, 256, 0, st>>>(static_cast<const float *>(src), src_proj_stride,
-                                                         src_row_stride, nproj, height, width, dark, flat_dark,
-                                                         field_row_stride, apply_log, dst, dst_proj_stride,
-                                                         dst_row_stride, nonpos);
+      launch_flat_log<float>(src, src_proj_stride, src_row_stride, nproj, height, width, chunk, dark, flat_dark,
+                             field_row_stride, apply_log, dst, dst_proj_stride, dst_row_stride, nonpos, st);
       break;
     case ATB_U16:
-      flat_log_kernel<unsigned short><<<(int)blocks, 256, 0, st>>>(
-          static_cast<const unsigned short *>(src), src_proj_stride, src_row_stride, nproj, height, width, dark,
-          flat_dark, field_row_stride, apply_log, dst, dst_proj_stride, dst_row_stride, nonpos);
+      launch_flat_log<unsigned short>(src, src_proj_stride, src_row_stride, nproj, height, width, chunk, dark,
+                                      flat_dark, field_row_stride, apply_log, dst, dst_proj_stride, dst_row_stride,
+                                      nonpos, st);
       break;
     default:
       return atb::fail(ATB_EINVAL, "atb_flat_log: unsupported src_dtype %d", src_dtype);
   }
   return atb::check_launch("atb_flat_log");
+}
+
+extern "C" int atb_flat_log(const void *src, int src_dtype, int64_t src_proj_stride, int64_t src_row_stride,
+                            int nproj, int height, int width, const float *dark, const float *flat_dark,
+                            int64_t field_row_stride, int apply_log, float *dst, int64_t dst_proj_stride,
+                            int64_t dst_row_stride, unsigned *nonpos, void *stream) {
+  return atb_flat_log_chunks(src, src_dtype, src_proj_stride, src_row_stride, nproj, height, width,
+                             nproj < 1 ? 1 : nproj, dark, flat_dark, field_row_stride, apply_log, dst,
+                             dst_proj_stride, dst_row_stride, nonpos, stream);
 }

@@ -6,7 +6,7 @@ Same names, signatures, defaults, errors and warnings as
 vertical reconstructions (``:450-1252``); the compute runs in the sm_100a
 kernels of ``libalgotom_b200.so``:
 
-- ``atb_flat_log``: flat/dark correction and ``-log`` of each chunk of
+- ``atb_flat_log_chunks``: flat/dark correction and ``-log`` of each chunk of
   projections (the reference's warning texts, and its in-place repair of
   values <= 0 in the caller's array when no flat field is given);
 - ``atb_filter_rows``: the ramp filter of every projection row
@@ -152,10 +152,12 @@ def _backproject(proj, trig, pts, center, edge_pad, acc):
              int(nbytes), R._stream_ptr(proj.device))
 
 
-def _flat_log(raw, code, dark, flat_dark, apply_log, out, nonpos):
+def _flat_log(raw, code, dark, flat_dark, apply_log, out, nonpos, chunk):
+    """The pre-step of every ``chunk`` projections, in one launch; one counter
+    of ``nonpos`` per chunk."""
     n, height, width = raw.shape
-    nat.call("atb_flat_log", raw.data_ptr(), code, raw.stride(0),
-             raw.stride(1), n, height, width,
+    nat.call("atb_flat_log_chunks", raw.data_ptr(), code, raw.stride(0),
+             raw.stride(1), n, height, width, chunk,
              dark.data_ptr() if dark is not None else None,
              flat_dark.data_ptr() if flat_dark is not None else None,
              dark.stride(0) if dark is not None else 0, int(bool(apply_log)),
@@ -618,16 +620,16 @@ def _reconstruct(projections, x_mat, y_mat, center, geo, flat_field,
                     tmp = torch.empty_like(pre)
                     work[("tmp", n)] = tmp
                 if code != nat.F32:  # counts to float32 first
-                    _flat_log(raw, code, None, None, False, pre, nonpos[:1])
+                    _flat_log(raw, code, None, None, False, pre, nonpos[:1],
+                              n)
                     raw = pre
                 _gaussian_slab(raw, wts, tmp, pre, to_int)
                 raw, code = pre, nat.F32
-            for k in range(k0, k1):  # one warning counter per chunk
-                if raw is pre and not apply_log and dark is None:
-                    break  # smoothed, nothing else to do
-                a, b = spans[k][0] - s0, spans[k][1] - s0
-                _flat_log(raw[a:b], code, dark, flat_dark, apply_log,
-                          pre[a:b], nonpos[k:k + 1])
+            if raw is not pre or apply_log or dark is not None:
+                # (else smoothed, nothing else to do); one warning counter
+                # per chunk
+                _flat_log(raw, code, dark, flat_dark, apply_log, pre,
+                          nonpos[k0:k1], chunk_size)
         src = pre
         if ramp_filter == "before":
             filt = work.get(("filt", n))

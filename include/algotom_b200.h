@@ -615,6 +615,18 @@ int atb_flat_log(const void *src, int src_dtype, int64_t src_proj_stride,
                  int64_t dst_proj_stride, int64_t dst_row_stride,
                  unsigned *nonpos, void *stream);
 
+/*
+ * The same for several chunks of `chunk` projections (the last one may be
+ * shorter) in one launch; nonpos[c] counts chunk c's replaced values.
+ */
+int atb_flat_log_chunks(const void *src, int src_dtype,
+                        int64_t src_proj_stride, int64_t src_row_stride,
+                        int nproj, int height, int width, int chunk,
+                        const float *dark, const float *flat_dark,
+                        int64_t field_row_stride, int apply_log, float *dst,
+                        int64_t dst_proj_stride, int64_t dst_row_stride,
+                        unsigned *nonpos, void *stream);
+
 /* ---------------------------------------------------------------------- */
 /* 360-degree sinograms (algotom/prep/conversion.py)                      */
 /* ---------------------------------------------------------------------- */
