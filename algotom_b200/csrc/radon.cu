@@ -87,7 +87,11 @@ __device__ __forceinline__ double walk_bin(const float *src, long long rs, int v
   const float rf = (float)r;
   const double ic = 0.5 * (double)(ncol - 1);
   double acc = 0.0;
-  const float c2 = 2.0f * cf, c3 = 3.0f * cf;
+  // weights of the three pixels from e = floor(u - span) - (u - span) in
+  // (-1, 0] and c = |cos| = 1 / span: their distances from the ray, in bins, are
+  // 1 - c - e c, |2 c - 1 + e c| and 3 c - 1 + e c (the first and the last keep
+  // their signs), so c + e c, 1 - |2 c - 1 + e c| and max(0, 2 - 3 c - e c)
+  const float c = fabsf(cf), c21 = fmaf(2.0f, c, -1.0f), c23 = fmaf(-3.0f, c, 2.0f);
   for (int va = v0; va < v1; va += kRun) {
     const double X0 = fma((double)va, r, A);
     const double xid = floor(X0);
@@ -103,22 +107,20 @@ __device__ __forceinline__ double walk_bin(const float *src, long long rs, int v
       const float xe = fmaf((float)(kRun - 1), rf, xf);  // xr is monotonic in j
       if (nrun == kRun && xi + floor_small(fminf(xf, xe) - spanf) + 1 >= 0 &&
           xi + floor_small(fmaxf(xf, xe) - spanf) + 3 <= ncol - 1) {
-        const float *base = line + xi;
+        const float *base = line + xi - 0x4B400000ll + 1;
+        const float xs = xf - spanf;
+        float run2 = 0.0f, run3 = 0.0f;
 #pragma unroll 8
         for (int j = 0; j < kRun; ++j, base += rs) {
-          const float xr = fmaf((float)j, rf, xf);
-          const float tq = __fadd_rd(xr - spanf, 12582912.0f);
-          const int xb = __float_as_int(tq) - 0x4B400000;
-          const float d0 = (tq - 12582912.0f) - xr;  // floor(xr - span) - xr
-          const float *px = base + xb;
-          const float w1 = fmaxf(0.0f, 1.0f - fabsf(fmaf(d0, cf, cf)));
-          const float w2 = fmaxf(0.0f, 1.0f - fabsf(fmaf(d0, cf, c2)));
-          const float w3 = fmaxf(0.0f, 1.0f - fabsf(fmaf(d0, cf, c3)));
-          run = fmaf(w1, __ldg(px + 1), run);
-          run = fmaf(w2, __ldg(px + 2), run);
-          run = fmaf(w3, __ldg(px + 3), run);
+          const float t = fmaf((float)j, rf, xs);
+          const float tq = __fadd_rd(t, 12582912.0f);  // 0x4B400000 + floor(t) as an integer
+          const float e = (tq - 12582912.0f) - t;
+          const float *px = base + __float_as_int(tq);
+          run = fmaf(fmaf(e, c, c), __ldg(px), run);
+          run2 = fmaf(1.0f - fabsf(fmaf(e, c, c21)), __ldg(px + 1), run2);
+          run3 = fmaf(fmaxf(0.0f, fmaf(-e, c, c23)), __ldg(px + 2), run3);
         }
-        acc += (double)run;
+        acc += (double)(run + (run2 + run3));
         continue;
       }
     }
