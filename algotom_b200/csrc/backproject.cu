@@ -58,7 +58,7 @@
 #include <cuda.h>  // CUtensorMap and its enums (the encoder is fetched at run time)
 #include <cudaTypedefs.h>
 
-#include <cmath>
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
@@ -1029,31 +1029,37 @@ __global__ void __launch_bounds__(256) sum_groups_kernel(BPArgs a) {
 }
 
 // Angles per CTA when a launch's tiles do not fill the GPU evenly: nrow (no
-// groups), or a multiple of the chunk.  A wave of CTAs takes as long as its
-// angles and about 40 more (prologue, epilogue); the sum of n groups' partial
-// images costs their traffic and a launch, in units of the 0.3 us that a wave
-// takes for an angle.  Tiles outside the inscribed disc are counted as empty
-// (they are with the default mask).
+// groups), or a multiple of the chunk.  The rule is read off a sweep of 1 to 24
+// groups (us; masked disc, sum of the groups included), whose optima are broad:
+//   64 x 64, one slice   1200 x 1536: 1155 (1), 970 (6), 935 (8), 974 (24)
+//                        1801 x 2560: 3755 (1), 3355 (6), 3462 (16)
+//   32 x 32, one slice   181 x 256: 75 (1), 48 (6); 400 x 400: 144 (1), 86 (6),
+//                        75 (13); 900 x 512: 290 (1), 178 (6), 161 (15);
+//                        900 x 1024: 521 (1), 453 (5), 446 (10), 466 (16);
+//                        900 x 1300: 751 (1), 670 (6), 717 (16)
+//   two slices           900 x 512: 430 (1), 234 (10); x 1024: 856 (1), 681 (6)
+//   four slices          300 x 300: 218 (1), 88 (8); 900 x 800: 744 (1), 705 (6)
+//   eight (two CTA layers of four): 900 x 1024: 1996 (1), 2018 (4)
 template <typename T, int S, int V>
 int group_rows(int nrow, int nslices, int ncol) {
   using K = BPCfg<T, S, V>;
-  const double tiles = 0.785 * ((ncol + K::TX - 1) / K::TX) * (double)((ncol + K::TY - 1) / K::TY) * ((nslices + S - 1) / S);
-  const double slots = 148.0 * K::kMinBlocks;
+  const long long tiles =
+      (long long)((ncol + K::TX - 1) / K::TX) * ((ncol + K::TY - 1) / K::TY) * ((nslices + S - 1) / S);
   const int nchunk = (nrow + K::kChunk - 1) / K::kChunk;
-  double best = 0.0;
-  int rows = nrow;
-  for (int g = 1; g <= 32 && g <= nchunk; ++g) {
-    const int r = (nchunk + g - 1) / g * K::kChunk, n = (nrow + r - 1) / r;
-    if (g > 1 && n != g) continue;
-    double cost = ceil(tiles * n / slots) * ((n > 1 ? r : nrow) + 40.0);
-    if (n > 1) cost += 13.0 + (double)ncol * ncol * nslices * n * 16.0 / 1.2e6;
-    if (g == 1 || cost < 0.95 * best) {
-      best = cost;
-      rows = n > 1 ? r : nrow;
-    }
-  }
-  return rows;
+  long long g;
+  if (S == 1 && V == 1) g = tiles > 3000 ? 1 : std::min(16ll, std::max(5ll, 11000 / tiles));
+  else if (S == 1) g = tiles > 3000 ? 1 : std::min(12ll, std::max(6ll, 4500 / tiles));
+  else if (S == 2) g = tiles > 1500 ? 1 : std::min(10ll, std::max(4ll, 4500 / tiles));
+  else g = tiles > 600 ? 1 : std::min(8ll, 2000 / tiles);
+  g = std::min(g, (long long)nchunk);
+  return g <= 1 ? nrow : (int)((nchunk + g - 1) / g * K::kChunk);
 }
+// The tile variant of a single slice that may be split: the one that is faster
+// unsplit (900 x 1300: 811 us in 64 x 64 tiles, 751 in 32 x 32 ones; 1200 x 1536:
+// 1155 and 1285).  Split, the larger tiles win from 700 pixels on (900 x 1024:
+// 400 and 446), but their FP32 positions are further from the tile's middle and
+// less exact (5.4e-7 against 4.7e-7 of error at 900 x 1024).
+int split_variant(int ncol) { return ncol < 1400 ? 1 : 0; }
 
 template <typename T, int S, bool kPerAngleKahan, int V = 0, bool kGroup = false>
 int launch_bp(BPArgs a, int nslices, cudaStream_t st, float2 *work = nullptr) {
@@ -1099,7 +1105,7 @@ int launch_bp(BPArgs a, int nslices, cudaStream_t st, float2 *work = nullptr) {
 template <typename T>
 int dispatch(BPArgs a, int per_angle_kahan, int variant, cudaStream_t st, float2 *work) {
   if (per_angle_kahan) return launch_bp<T, 1, true>(a, a.nslice, st);
-  if (work) variant = 1;  // (the smaller tiles split better)
+  if (work) variant = split_variant(a.ncol);
   if (a.nslice == 1 && variant == 1) return launch_bp<T, 1, false, 1>(a, 1, st, work);
   // four slices per CTA for the bulk of a stack, then the remainder
   const int n4 = (a.nslice / 4) * 4;
@@ -1115,7 +1121,7 @@ int dispatch(BPArgs a, int per_angle_kahan, int variant, cudaStream_t st, float2
     a.slice_base = n4 + 2;
   }
   if (variant == 1) return launch_bp<T, 1, false, 1>(a, 1, st, work);
-  return launch_bp<T, 1, false>(a, 1, st);
+  return launch_bp<T, 1, false>(a, 1, st, work);
 }
 
 // bytes of the partial images of dispatch's largest launch; 0 without groups
@@ -1129,7 +1135,8 @@ long long split_bytes(int nrow, int nslice, int ncol) {
   const int n4 = (nslice / 4) * 4, rem = nslice - n4;
   if (n4 > 0) add(group_rows<T, 4, 0>(nrow, n4, ncol), n4);
   if (rem >= 2) add(group_rows<T, 2, 0>(nrow, 2, ncol), 2);
-  if (rem & 1) add(group_rows<T, 1, 1>(nrow, 1, ncol), 1);
+  if (rem & 1)
+    add(split_variant(ncol) ? group_rows<T, 1, 1>(nrow, 1, ncol) : group_rows<T, 1, 0>(nrow, 1, ncol), 1);
   return need;
 }
 
