@@ -19,23 +19,29 @@
 namespace atb {
 namespace dfi {
 
-// centred quintic B-spline
-__device__ __forceinline__ double bspline5(double u) {
-  const double a = fabs(u);
-  if (a < 1.0) {
+// The six weights of the centred quintic B-spline at distances t + 2, t + 1, t,
+// 1 - t, 2 - t and 3 - t, 0 <= t < 1: its three polynomials, each where it
+// holds, without branches or divisions (which took most of the FP64 work of a
+// point).
+__device__ __forceinline__ void bspline5_weights(double t, double (&w)[6]) {
+  auto inner = [](double a) {  // a < 1
     const double a2 = a * a;
-    return 11.0 / 20.0 - a2 / 2.0 + a2 * a2 / 4.0 - a2 * a2 * a / 12.0;
-  }
-  if (a < 2.0) {
-    const double a2 = a * a;
-    return 17.0 / 40.0 + 5.0 * a / 8.0 - 7.0 * a2 / 4.0 + 5.0 * a2 * a / 4.0 - 3.0 * a2 * a2 / 8.0 +
-           a2 * a2 * a / 24.0;
-  }
-  if (a < 3.0) {
-    const double b = 3.0 - a, b2 = b * b;
-    return b2 * b2 * b / 120.0;
-  }
-  return 0.0;
+    return fma(a2, fma(a2, fma(a, -1.0 / 12.0, 0.25), -0.5), 0.55);
+  };
+  auto middle = [](double a) {  // 1 <= a < 2
+    return fma(a, fma(a, fma(a, fma(a, fma(a, 1.0 / 24.0, -0.375), 1.25), -1.75), 0.625), 0.425);
+  };
+  auto outer = [](double b) {  // b = 3 - a
+    const double b2 = b * b;
+    return b2 * b2 * b * (1.0 / 120.0);
+  };
+  const double s = 1.0 - t;
+  w[0] = outer(s);
+  w[1] = middle(1.0 + t);
+  w[2] = inner(t);
+  w[3] = inner(s);
+  w[4] = middle(1.0 + s);
+  w[5] = outer(t);
 }
 
 // half-sample symmetric index
@@ -62,13 +68,14 @@ __device__ __forceinline__ double2 regrid_point(const double2 *__restrict__ coef
   if (th > M_PI) th -= M_PI;
   const float tf = (float)(th * (nrow - 1.0) / M_PI);
   const double rr = (double)tf, cc = (double)r;
-  const int fr = (int)floor(rr) - 2, fc = (int)floor(cc) - 2;
+  const double rf = floor(rr), cf = floor(cc);
+  const int fr = (int)rf - 2, fc = (int)cf - 2;
   double wr[6], wc[6];
+  bspline5_weights(rr - rf, wr);
+  bspline5_weights(cc - cf, wc);
   int ir[6], ic[6];
 #pragma unroll
   for (int m = 0; m < 6; ++m) {
-    wr[m] = bspline5(rr - (fr + m));
-    wc[m] = bspline5(cc - (fc + m));
     ir[m] = reflect_index(fr + m, nrow);
     ic[m] = reflect_index(fc + m, w);
   }
