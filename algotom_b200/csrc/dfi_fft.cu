@@ -60,6 +60,9 @@ struct Tables {
 template <bool INV>
 __device__ void bluestein(double2 *x, int w, const IpPlan &pl, const double2 *tws, const Tables &t) {
   const int M = pl.n;
+  // M is a power of two, so the lanes of a warp that take part in a step are all,
+  // or the first M
+  const unsigned lanes = M >= 32 ? 0xffffffffu : (1u << M) - 1u;
   // into the transform's order: elements move within aligned groups of eight,
   // which lie in one warp's hands
   for (int n = threadIdx.x; n < M; n += blockDim.x) {
@@ -68,7 +71,7 @@ __device__ void bluestein(double2 *x, int w, const IpPlan &pl, const double2 *tw
       const double2 b = __ldg(t.chirp + n);
       v = INV ? cmul(x[n], b) : cmulc(x[n], b);
     }
-    __syncwarp(__activemask());
+    __syncwarp(lanes);
     x[ip_at(n)] = v;
   }
   __syncthreads();
@@ -83,7 +86,7 @@ __device__ void bluestein(double2 *x, int w, const IpPlan &pl, const double2 *tw
       const double2 b = __ldg(t.chirp + k);
       v = INV ? cmul(v, b) : cmulc(v, b);
     }
-    __syncwarp(__activemask());
+    __syncwarp(lanes);
     x[k] = v;
   }
   __syncthreads();
