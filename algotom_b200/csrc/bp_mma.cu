@@ -49,13 +49,14 @@
 // - four warps read each tile's sums, zero them and keep the compensated
 //   totals, in registers that the other warps give up.
 // The tiles' sums end in turn, so that one tile's read is covered by the
-// others' MMAs.  What bounds it: the weight warps' issue (about 27 instructions
-// per row, 65 % of all issue slots taken, the integer pipe 53 %), which is why
-// the cost of a launch hardly depends on the number of slices; the tensor
-// cores are busy 40 % of the time.
-// Measured, 1801 angles of 2560 bins, 32 slices, no mask: 56.6 ms against
-// 103 ms with the gather kernel (6.7e12 and 3.7e12 updates/s); 901 x 1280:
-// 6.3 against 10.2 ms with 24 slices, 6.1 against 6.9 with 16.
+// others' MMAs.  What bounds it: the weight warps' issue (72 % of all issue slots
+// taken, the integer pipe 57 %), which is why the cost of a launch hardly depends
+// on the number of slices; the tensor cores are busy 45 % of the time.  Under
+// sustained load the power cap sets the clock (1.70 GHz).
+// Measured, 1801 angles of 2560 bins, 32 slices, no mask: 53.9 ms against
+// 100.5 ms with the gather kernel (7.0e12 and 3.8e12 updates/s); 901 x 1024: 4.14
+// against 8.68; 901 x 1280: 6.16 against 10.03 ms with 24 slices, 6.23 against
+// 6.76 with 16.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -623,7 +624,13 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
   }
   fence_before();
   __syncthreads();
-  if (tid == 0 && *bad) atomicOr(&g_mma_status, 1);
+  if (*bad) {
+    if (tid == 0) atomicOr(&g_mma_status, 1);
+    // copies and MMAs that are still in flight end in microseconds; this CTA's
+    // memory is its own for another millisecond
+    for (int n = 0; n < 64; ++n) __nanosleep(16000);
+    __syncthreads();
+  }
   if (!*bad && tid < 3 * kRegion * kRegion) {
     // thread = pixel of the region, and every third slice
     const int xr = tid & (kRegion - 1), yr = (tid / kRegion) & (kRegion - 1);
