@@ -41,6 +41,8 @@ FLOP_PER_UPDATE = 7.0
 # on-chip bytes one update must read: the two FP32 taps of its bin (held as
 # one 8-byte interpolation pair in shared memory)
 SMEM_BYTES_PER_UPDATE = 8.0
+# tensor-core back-projector: 2 weight terms x 2 sample terms x 16 bins x 2
+MMA_FLOP_PER_UPDATE = 128.0
 SMEM_BYTES_PER_CLK_PER_SM = 128.0
 N_SM = 148
 
@@ -155,14 +157,14 @@ class ClockSampler:
                 "samples": len(sm), "reasons": sorted(reasons)}
 
 
-TRAFFIC_PROFILE = "profiles/backproject_c2_16slices.md"
+TRAFFIC_PROFILE = "profiles/bp_mma_c2_32slices.md"
 
 
 def _traffic_per_update():
     """DRAM bytes per update of the back-projection kernel as an ncu capture
     measured them: the `dram_bytes_per_update:` line of the committed
     summary TRAFFIC_PROFILE (dram__bytes_read.sum + dram__bytes_write.sum of
-    one launch on 16 slices, divided by its updates; the bench cannot read
+    one launch on 32 slices, divided by its updates; the bench cannot read
     DRAM counters itself).  Returns (bytes per update, the summary's
     `build:` line) or (None, None)."""
     try:
@@ -459,10 +461,15 @@ def run_ours(args, rank, world, local_rank):
     peaks, src = _peaks()
     f_clk = float(peaks.get("sm_max_mhz", 1965.0)) * 1e6
     fp32_peak = 2.0 * 128 * N_SM * f_clk / 1e12          # TFLOP/s
-    smem_peak = SMEM_BYTES_PER_CLK_PER_SM * N_SM * f_clk / 1e9  # GB/s
     bp_upd = nslice * NCOL * NCOL * NROW
     achieved = FLOP_PER_UPDATE * bp_upd / t_bp / 1e12
-    smem_achieved = SMEM_BYTES_PER_UPDATE * bp_upd / t_bp / 1e9
+    # products of the tensor-core back-projector: regions of 16 x 16 pixels
+    # that the circle mask leaves
+    edge = np.arange(0, NCOL, 16) - NCOL // 2
+    near = np.maximum(0, np.maximum(edge, -(edge + 15)))
+    live = float(np.mean(near[:, None] ** 2 + near[None] ** 2 <= mask_r2))
+    tensor_peak = float(peaks.get("bf16_tflops", 1590.0))
+    tensor_achieved = MMA_FLOP_PER_UPDATE * live * bp_upd / t_bp / 1e12
     tpu, tbuild = _traffic_per_update()
     filt_bytes = NROW * nslice * NCOL * 8.0
     line = {
@@ -477,15 +484,17 @@ def run_ours(args, rank, world, local_rank):
                    "l2": "inputs larger than L2 (4.7 GB sinogram per GPU)"},
         "slices_per_s": world * nslice * args.steps / t_dev,
         "accuracy": err,
-        "roofline": {"bound": "smem", "kernel": "bp_kernel",
-                     "achieved": smem_achieved, "peak": smem_peak,
-                     "unit": "GB/s", "frac": smem_achieved / smem_peak,
+        "roofline": {"bound": "tensor", "kernel": "bp_mma_kernel",
+                     "achieved": tensor_achieved, "peak": tensor_peak,
+                     "unit": "TFLOP/s", "frac": tensor_achieved / tensor_peak,
                      "traffic": (tpu * bp_upd if tpu else None),
-                     "bytes_per_update": SMEM_BYTES_PER_UPDATE,
+                     "flop_per_update": MMA_FLOP_PER_UPDATE,
+                     "live_fraction": live,
                      "updates_per_s": bp_upd / t_bp,
                      "ms_per_launch": t_bp * 1e3,
-                     "peak_source": "shared-memory delivery, 128 B/clk x 148 "
-                                    "SM x sm_max_mhz (%s)" % src,
+                     "peak_source": "float16 tensor cores, the measured bf16 "
+                                    "GEMM burst (%s); regions outside the "
+                                    "circle mask do no products" % src,
                      "traffic_source": ("ncu dram__bytes_read.sum + "
                                         "dram__bytes_write.sum per update "
                                         "from %s (%s), times this launch's "
@@ -507,7 +516,9 @@ def run_ours(args, rank, world, local_rank):
         "cpu_baseline": cpu,
         "e2e": e2e,
         "batch": batch,
-        "gpu_launches": 2 * args.steps,
+        # the filter, and per 32 slices the scan, the packing, the
+        # tensor-core back-projection and the gated gather kernel
+        "gpu_launches": (1 + 4 * -(-nslice // 32)) * args.steps,
         "clocks": clocks,
     }
     print(json.dumps(line), flush=True)
@@ -995,6 +1006,10 @@ def _group_launches(CC, centers):
         return 1
     n = 0
     for _, _, _, _, cnt in groups:
+        if cnt >= 15:  # tensor cores: a scan, then packing, the products and
+            # the ring of blocks per 32 centres; below 15 as the rest
+            n += 1 + 3 * (cnt // 32 + int(cnt % 32 >= 15))
+            cnt = cnt % 32 if cnt % 32 < 15 else 0
         rem = cnt % 4
         n += int(cnt >= 4) + int(rem >= 2) + int(rem % 2)
     return n
