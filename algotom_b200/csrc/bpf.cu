@@ -34,6 +34,7 @@
 // The ramp amplifies rounding of the smooth back-projection by about 140x
 // at 2560^2, which is why the transforms run in FP64 (FP32 gave 2.2e-5
 // relative L2 against the FP64 oracle).
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 
@@ -123,11 +124,29 @@ __device__ double pad_value(const BpfArgs &a, const float *X, int ks, int ry, in
   }
 }
 
+// Threads of an SM for the 2-D filter's kernels, all its CTAs together: without
+// the radices 11 and 13 (BIG) a butterfly lives in 80 registers, with them in
+// 128.  Stages are bound by latency (shared memory, FP64) and by shared-memory
+// bandwidth, so a transform takes as many warps as the registers allow, and its
+// first read, the product with the spectrum and its last write ride on its
+// stages instead of passing over shared memory.  16 slices, ms, before (256
+// threads of 98 registers, every twiddle looked up, those passes); now with 128 /
+// 256 / 384 threads:
+//   T 588: 0.199; 0.110 / 0.151 / 0.192    1176: 0.696; 0.413 / 0.447 / 0.570
+//   T 1536: 1.667; 1.170 / 0.978 / 1.191   2048: 2.811; 2.353 / 2.034 / 2.075
+//   T 2352: 2.911; 2.359 / 1.934 / 1.784   2880: 3.821; 3.241 / 2.651 / 2.488
+//   T 4410: 13.72; 14.14 / 9.93 / 8.78, 768: 8.09
+// and with the radices 11 and 13 (128 / 256): 1300: 1.165; 0.727 / 0.951; 2860:
+// 5.086; 4.942 / 3.859.  So few threads while five CTAs and more fit, else as many
+// as fill the register file.
+constexpr int fft_threads(bool big) { return big ? 512 : 768; }
+
 // Grids put the slice pair on x, so that the CTAs of one row / column of
 // every pair run together (the columns kernel then reads each spectrum
 // column once from DRAM).  Shared memory: two buffers of T values, then
 // the twiddle table.
-__global__ void __launch_bounds__(kThreads) bpf_rows_kernel(BpfArgs a, const __grid_constant__ Plan pl) {
+template <bool BIG>
+__global__ void __launch_bounds__(fft_threads(BIG), 1) bpf_rows_kernel(BpfArgs a, const __grid_constant__ Plan pl) {
   extern __shared__ double2 sm[];
   const int ry = blockIdx.y, g = blockIdx.x, T = pl.n;
   double2 *tws = sm + 2 * T;
@@ -145,47 +164,52 @@ __global__ void __launch_bounds__(kThreads) bpf_rows_kernel(BpfArgs a, const __g
     sm[rx] = z;
   }
   __syncthreads();
-  const double2 *res = atb::fft::run<false>(sm, sm + T, pl, tws);
   double2 *w = a.work + ((long long)g * a.n + ry) * T;
-  for (int kx = threadIdx.x; kx < T; kx += blockDim.x) w[kx] = res[kx];
+  atb::fft::run_io<false, BIG>(sm, sm + T, pl, tws, atb::fft::FromBuffer(),
+                               [w](double2 *, int kx, double2 v) { w[kx] = v; });
 }
 
-__global__ void __launch_bounds__(kThreads) bpf_cols_kernel(BpfArgs a, const __grid_constant__ Plan pl) {
+template <bool BIG>
+__global__ void __launch_bounds__(fft_threads(BIG), 1) bpf_cols_kernel(BpfArgs a, const __grid_constant__ Plan pl) {
   extern __shared__ double2 sm[];
   const int kx = blockIdx.y, g = blockIdx.x, T = pl.n, n = a.n;
   double2 *tws = sm + 2 * T;
   atb::fft::load_twiddles(pl, tws);
   double2 *w = a.work + (long long)g * n * T + kx;
-  for (int ry = threadIdx.x; ry < T; ry += blockDim.x)
-    sm[ry] = ry < n ? w[(long long)ry * T] : make_double2(0.0, 0.0);
   __syncthreads();
-  double2 *res = atb::fft::run<false>(sm, sm + T, pl, tws);
-  double2 *other = res == sm ? sm + T : sm;
-  if (a.spec_complex) {
-    const double2 *S = static_cast<const double2 *>(a.spec) + (long long)kx * T;
-    for (int ky = threadIdx.x; ky < T; ky += blockDim.x) res[ky] = atb::fft::cmul(res[ky], __ldg(S + ky));
-  } else {
-    const double *S = static_cast<const double *>(a.spec) + (long long)kx * T;
-    for (int ky = threadIdx.x; ky < T; ky += blockDim.x) {
-      const double h = __ldg(S + ky);
-      res[ky].x *= h;
-      res[ky].y *= h;
-    }
-  }
-  __syncthreads();
-  const double2 *out = atb::fft::run<true>(res, other, pl, tws);
-  for (int u = a.pad + threadIdx.x; u < a.pad + a.ncol; u += blockDim.x) w[(long long)u * T] = out[u];
+  const bool cplx = a.spec_complex;
+  const double2 *Sc = static_cast<const double2 *>(a.spec) + (long long)kx * T;
+  const double *Sr = static_cast<const double *>(a.spec) + (long long)kx * T;
+  double2 *res = atb::fft::run_io<false, BIG>(
+      sm, sm + T, pl, tws,
+      [w, n, T](const double2 *, int ry) { return ry < n ? w[(long long)ry * T] : make_double2(0.0, 0.0); },
+      [cplx, Sc, Sr](double2 *buf, int ky, double2 v) {
+        if (cplx) {
+          v = atb::fft::cmul(v, __ldg(Sc + ky));
+        } else {
+          const double h = __ldg(Sr + ky);
+          v.x *= h;
+          v.y *= h;
+        }
+        buf[ky] = v;
+      });
+  const int u0 = a.pad, u1 = a.pad + a.ncol;
+  atb::fft::run_io<true, BIG>(res, res == sm ? sm + T : sm, pl, tws, atb::fft::FromBuffer(),
+                              [w, T, u0, u1](double2 *, int u, double2 v) {
+                                if (u >= u0 && u < u1) w[(long long)u * T] = v;
+                              });
 }
 
-__global__ void __launch_bounds__(kThreads) bpf_out_kernel(BpfArgs a, const __grid_constant__ Plan pl) {
+template <bool BIG>
+__global__ void __launch_bounds__(fft_threads(BIG), 1) bpf_out_kernel(BpfArgs a, const __grid_constant__ Plan pl) {
   extern __shared__ double2 sm[];
   const int y = blockIdx.y, g = blockIdx.x, T = pl.n;
   double2 *tws = sm + 2 * T;
   atb::fft::load_twiddles(pl, tws);
   const double2 *w = a.work + ((long long)g * a.n + y + a.pad) * T;
-  for (int kx = threadIdx.x; kx < T; kx += blockDim.x) sm[kx] = w[kx];
   __syncthreads();
-  const double2 *res = atb::fft::run<true>(sm, sm + T, pl, tws);
+  const double2 *res = atb::fft::run_io<true, BIG>(
+      sm, sm + T, pl, tws, [w](const double2 *, int kx) { return w[kx]; }, atb::fft::ToBuffer());
   const int sa = a.slice0 + 2 * g, sb = sa + 1;
   const bool hb = sb < a.nslice;
   const int c = a.ncol / 2;
@@ -585,9 +609,19 @@ extern "C" int atb_bpf_filter2d(const float *src, int64_t src_row_stride, int64_
     ++pairs;
 
   const size_t smem = (2 * (size_t)t + atb::fft::twiddle_entries(t)) * sizeof(double2);
-  int rc = atb::ensure_smem(bpf_rows_kernel, smem, "atb_bpf_filter2d");
-  if (rc == ATB_OK) rc = atb::ensure_smem(bpf_cols_kernel, smem, "atb_bpf_filter2d");
-  if (rc == ATB_OK) rc = atb::ensure_smem(bpf_out_kernel, smem, "atb_bpf_filter2d");
+  bool big = false;
+  for (int k = 0; k < pl.nstages; ++k) big = big || pl.radix[k] > 8;
+  // the CTAs of an SM share its threads: of 128 where the shared memory holds five
+  // and more (four, BIG), else three (two), two or one
+  const int fit = (int)std::max<size_t>(1, 228 * 1024 / (smem + 1024));
+  const int ctas = big ? (fit >= 4 ? 4 : std::min(2, fit)) : (fit >= 5 ? 6 : std::min(3, fit));
+  const int threads = fft_threads(big) / ctas;
+  const auto rows = big ? bpf_rows_kernel<true> : bpf_rows_kernel<false>;
+  const auto cols = big ? bpf_cols_kernel<true> : bpf_cols_kernel<false>;
+  const auto outs = big ? bpf_out_kernel<true> : bpf_out_kernel<false>;
+  int rc = atb::ensure_smem(rows, smem, "atb_bpf_filter2d");
+  if (rc == ATB_OK) rc = atb::ensure_smem(cols, smem, "atb_bpf_filter2d");
+  if (rc == ATB_OK) rc = atb::ensure_smem(outs, smem, "atb_bpf_filter2d");
   int m2 = 1;  // the median sorts a power-of-two line
   while (m2 < ncol) m2 <<= 1;
   const size_t stat_smem = (size_t)m2 * sizeof(double);
@@ -627,9 +661,9 @@ extern "C" int atb_bpf_filter2d(const float *src, int64_t src_row_stride, int64_
       bpf_stats_kernel<<<dim3(2 * ncol, gs), kStatThreads, 0, st>>>(a, colstat, rowstat);
       bpf_padstat_kernel<<<gs, kStatThreads, stat_smem, st>>>(a, colstat, padstat);
     }
-    bpf_rows_kernel<<<dim3(gp, n), kThreads, smem, st>>>(a, pl);
-    bpf_cols_kernel<<<dim3(gp, t), kThreads, smem, st>>>(a, pl);
-    bpf_out_kernel<<<dim3(gp, ncol), kThreads, smem, st>>>(a, pl);
+    rows<<<dim3(gp, n), threads, smem, st>>>(a, pl);
+    cols<<<dim3(gp, t), threads, smem, st>>>(a, pl);
+    outs<<<dim3(gp, ncol), threads, smem, st>>>(a, pl);
     rc = atb::check_launch("atb_bpf_filter2d");
     if (rc != ATB_OK) return rc;
   }

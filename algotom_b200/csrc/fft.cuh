@@ -147,9 +147,18 @@ __device__ __forceinline__ double2 twiddle(const double2 *tws, int e) {
   return cmul(tws[kTwLo + (e >> 6)], tws[e & (kTwLo - 1)]);
 }
 
-template <int P, bool INV>
+// How a stage reads and writes: from and to a buffer, unless the first or the
+// last stage of a transform is given something else (run_io).
+struct FromBuffer {
+  __device__ __forceinline__ double2 operator()(const double2 *buf, int i) const { return buf[i]; }
+};
+struct ToBuffer {
+  __device__ __forceinline__ void operator()(double2 *buf, int i, double2 v) const { buf[i] = v; }
+};
+
+template <int P, bool INV, typename In = FromBuffer, typename Out = ToBuffer>
 __device__ __forceinline__ void stage(const double2 *__restrict__ in, double2 *__restrict__ out, const Plan &pl,
-                                      const double2 *tws, int L) {
+                                      const double2 *tws, int L, const In &get = In(), const Out &put = Out()) {
   const int n = pl.n, m = n / P;
   const int tstep = n / (L * P);  // twiddle index step per unit of r * k
   // the odd radix's cos / sin in registers for the whole stage (read
@@ -165,7 +174,7 @@ __device__ __forceinline__ void stage(const double2 *__restrict__ in, double2 *_
     const int i = L > 1 ? (int)__umulhi((unsigned)j, magic) : j, k = j - i * L;
     double2 v[P];
 #pragma unroll
-    for (int r = 0; r < P; ++r) v[r] = in[j + r * m];
+    for (int r = 0; r < P; ++r) v[r] = get(in, j + r * m);
     if (k > 0) {
       // one table value and its powers: P - 1 look-ups of two values each
       // were two thirds of the stage's shared-memory traffic
@@ -178,10 +187,57 @@ __device__ __forceinline__ void stage(const double2 *__restrict__ in, double2 *_
       }
     }
     dft<P, INV>(v, rc);
-    double2 *o = out + i * L * P + k;
+    const int o = i * L * P + k;
 #pragma unroll
-    for (int q = 0; q < P; ++q) o[q * L] = v[q];
+    for (int q = 0; q < P; ++q) put(out, o + q * L, v[q]);
   }
+}
+
+// BIG: with the radices 11 and 13, whose butterflies need the most registers.
+template <bool INV, bool BIG, typename In, typename Out>
+__device__ __forceinline__ void stage_of(int p, const double2 *a, double2 *b, const Plan &pl, const double2 *tws, int L,
+                                         const In &get, const Out &put) {
+  switch (p) {
+    case 2: stage<2, INV>(a, b, pl, tws, L, get, put); break;
+    case 3: stage<3, INV>(a, b, pl, tws, L, get, put); break;
+    case 4: stage<4, INV>(a, b, pl, tws, L, get, put); break;
+    case 5: stage<5, INV>(a, b, pl, tws, L, get, put); break;
+    case 7: stage<7, INV>(a, b, pl, tws, L, get, put); break;
+    case 8: stage<8, INV>(a, b, pl, tws, L, get, put); break;
+    default:
+      if constexpr (BIG) {
+        if (p == 11) stage<11, INV>(a, b, pl, tws, L, get, put);
+        else stage<13, INV>(a, b, pl, tws, L, get, put);
+      }
+      break;
+  }
+}
+
+// run, whose first stage reads value i with get(a, i) and whose last stage
+// writes value i with put(buffer, i, value): what comes before and after a
+// transform then needs no pass of its own over shared memory.
+template <bool INV, bool BIG, typename In, typename Out>
+__device__ double2 *run_io(double2 *a, double2 *b, const Plan &pl, const double2 *tws, const In &get, const Out &put) {
+  int L = 1;
+  const int last = pl.nstages - 1;
+  if (last < 0) {  // one value
+    if (threadIdx.x == 0) put(b, 0, get(a, 0));
+    __syncthreads();
+    return b;
+  }
+  for (int s = 0; s <= last; ++s) {
+    const int p = pl.radix[s];
+    if (s == 0 && s == last) stage_of<INV, BIG>(p, a, b, pl, tws, L, get, put);
+    else if (s == 0) stage_of<INV, BIG>(p, a, b, pl, tws, L, get, ToBuffer());
+    else if (s == last) stage_of<INV, BIG>(p, a, b, pl, tws, L, FromBuffer(), put);
+    else stage_of<INV, BIG>(p, a, b, pl, tws, L, FromBuffer(), ToBuffer());
+    __syncthreads();
+    double2 *t = a;
+    a = b;
+    b = t;
+    L *= p;
+  }
+  return a;
 }
 
 // Transform of the n values in a[] (b[] is scratch of the same size; tws
@@ -191,22 +247,12 @@ template <bool INV>
 __device__ double2 *run(double2 *a, double2 *b, const Plan &pl, const double2 *tws) {
   int L = 1;
   for (int s = 0; s < pl.nstages; ++s) {
-    const int p = pl.radix[s];
-    switch (p) {
-      case 2: stage<2, INV>(a, b, pl, tws, L); break;
-      case 3: stage<3, INV>(a, b, pl, tws, L); break;
-      case 4: stage<4, INV>(a, b, pl, tws, L); break;
-      case 5: stage<5, INV>(a, b, pl, tws, L); break;
-      case 7: stage<7, INV>(a, b, pl, tws, L); break;
-      case 8: stage<8, INV>(a, b, pl, tws, L); break;
-      case 11: stage<11, INV>(a, b, pl, tws, L); break;
-      default: stage<13, INV>(a, b, pl, tws, L); break;
-    }
+    stage_of<INV, true>(pl.radix[s], a, b, pl, tws, L, FromBuffer(), ToBuffer());
     __syncthreads();
     double2 *t = a;
     a = b;
     b = t;
-    L *= p;
+    L *= pl.radix[s];
   }
   return a;
 }
