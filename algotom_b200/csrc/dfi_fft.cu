@@ -50,7 +50,7 @@ constexpr int kMaxM = 8192;  // one buffer of M complex doubles + twiddles in 22
 struct Tables {
   const double2 *chirp;  // [w] b_m = exp(i pi m^2 / w)
   const double2 *tw;     // [M] exp(-2 pi i m / M)
-  const double2 *bfwd;   // [M] forward transform of the chirp kernel / M (digit-reversed)
+  const double2 *bfwd;   // [M] forward transform of the chirp kernel / M (order of ip_table_at)
   const double2 *binv;   // [M] the same for the conjugate chirp
 };
 
@@ -75,11 +75,7 @@ __device__ void bluestein(double2 *x, int w, const IpPlan &pl, const double2 *tw
     x[ip_at(n)] = v;
   }
   __syncthreads();
-  atb::fft::ip_run<false>(x, pl, tws);
-  const double2 *B = INV ? t.binv : t.bfwd;
-  for (int p = threadIdx.x; p < M; p += blockDim.x) x[ip_at(p)] = cmul(x[ip_at(p)], __ldg(B + p));
-  __syncthreads();
-  atb::fft::ip_run<true>(x, pl, tws);
+  atb::fft::ip_convolve(x, pl, tws, INV ? t.binv : t.bfwd);
   for (int k = threadIdx.x; k < M; k += blockDim.x) {  // (whole groups of eight)
     double2 v = x[ip_at(k)];
     if (k < w) {
@@ -113,7 +109,8 @@ __global__ void __launch_bounds__(kThreads) chirp_setup_kernel(int w, const __gr
   atb::fft::ip_run<false>(sm, pl, tws);
   double2 *out = conj ? binv : bfwd;
   const double s = 1.0 / (double)M;
-  for (int p = threadIdx.x; p < M; p += blockDim.x) out[p] = make_double2(sm[ip_at(p)].x * s, sm[ip_at(p)].y * s);
+  for (int p = threadIdx.x; p < M; p += blockDim.x)
+    out[atb::fft::ip_table_at(pl, p)] = make_double2(sm[ip_at(p)].x * s, sm[ip_at(p)].y * s);
 }
 
 // ---- padding (np.pad(row, pad, mode), numpy's ten modes, float32)

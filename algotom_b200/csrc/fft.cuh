@@ -353,12 +353,14 @@ __device__ __forceinline__ void ip_stage(double2 *x, int n, int L, const double2
 }
 
 // Every thread of the CTA calls these; a barrier separates the stages and
-// follows the last one.  Element i is x[ip_at(i)] before and after.
-template <bool INV>
+// follows the last one.  Element i is x[ip_at(i)] before and after.  ALL: with
+// the stage on the smallest blocks (the forward transform's last, the inverse's
+// first).
+template <bool INV, bool ALL = true>
 __device__ void ip_run(double2 *x, const IpPlan &pl, const double2 *tws) {
   if constexpr (!INV) {
     int L = pl.n;
-    for (int s = 0; s < pl.nstages; ++s) {
+    for (int s = 0; s < pl.nstages - !ALL; ++s) {
       const int r = pl.radix[s];
       if (r == 8) ip_stage<8, false>(x, pl.n, L, tws);
       else if (r == 4) ip_stage<4, false>(x, pl.n, L, tws);
@@ -367,8 +369,8 @@ __device__ void ip_run(double2 *x, const IpPlan &pl, const double2 *tws) {
       L /= r;
     }
   } else {
-    int L = 1;
-    for (int s = pl.nstages - 1; s >= 0; --s) {
+    int L = ALL ? 1 : pl.radix[pl.nstages - 1];
+    for (int s = pl.nstages - 1 - !ALL; s >= 0; --s) {
       const int r = pl.radix[s];
       L *= r;
       if (r == 8) ip_stage<8, true>(x, pl.n, L, tws);
@@ -377,6 +379,58 @@ __device__ void ip_run(double2 *x, const IpPlan &pl, const double2 *tws) {
       __syncthreads();
     }
   }
+}
+
+// Where value p of a transform (digit-reversed order) sits in the table that
+// ip_convolve multiplies by: the values of one block apart, so that
+// neighbouring threads read neighbouring entries.
+__device__ __forceinline__ int ip_table_at(const IpPlan &pl, int p) {
+  const int r = pl.radix[pl.nstages - 1];
+  return (p & (r - 1)) * (pl.n / r) + p / r;
+}
+
+template <int R>
+__device__ __forceinline__ void ip_middle(double2 *x, int n, const double2 *__restrict__ B) {
+  const int nq = n / R, nt = blockDim.x;
+  for (int q0 = threadIdx.x; q0 < nq; q0 += 2 * nt) {
+    const int q1 = q0 + nt;
+    const bool two = q1 < nq;
+    double2 v0[R], v1[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      v0[j] = x[ip_at(q0 * R + j)];
+      v1[j] = two ? x[ip_at(q1 * R + j)] : make_double2(0.0, 0.0);
+    }
+    ip_butterfly<R, false>(v0, 0, 0, nullptr);
+    ip_butterfly<R, false>(v1, 0, 0, nullptr);
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      v0[j] = cmul(v0[j], __ldg(B + j * nq + q0));
+      if (two) v1[j] = cmul(v1[j], __ldg(B + j * nq + q1));
+    }
+    ip_butterfly<R, true>(v0, 0, 0, nullptr);
+    ip_butterfly<R, true>(v1, 0, 0, nullptr);
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      x[ip_at(q0 * R + j)] = v0[j];
+      if (two) x[ip_at(q1 * R + j)] = v1[j];
+    }
+  }
+}
+
+// Circular convolution with the kernel whose transform is B (in the order of
+// ip_table_at).  The forward transform's last stage and the inverse's first work
+// on the same blocks, so both and the product are one pass over shared memory
+// and one barrier where they were three (DFI of 901 x 1280, M = 4096: 607 ->
+// 572 us; of 1801 x 2560, M = 8192: 2.16 -> 2.01 ms).
+__device__ __forceinline__ void ip_convolve(double2 *x, const IpPlan &pl, const double2 *tws, const double2 *B) {
+  ip_run<false, false>(x, pl, tws);
+  const int r = pl.radix[pl.nstages - 1];
+  if (r == 8) ip_middle<8>(x, pl.n, B);
+  else if (r == 4) ip_middle<4>(x, pl.n, B);
+  else ip_middle<2>(x, pl.n, B);
+  __syncthreads();
+  ip_run<true, false>(x, pl, tws);
 }
 
 }  // namespace fft
