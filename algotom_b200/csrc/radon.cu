@@ -101,14 +101,14 @@ __device__ __forceinline__ double walk_bin(const float *src, long long rs, int v
     const float *line = src + (long long)va * rs;
     float run = 0.0f;
     if constexpr (!kEdge) {
-      // a full run whose candidate pixels all lie inside the line: no
-      // bounds logic, weights clamped at zero (a zero weight adds exactly 0,
-      // the same sum as the checked loop below)
-      const float xe = fmaf((float)(kRun - 1), rf, xf);  // xr is monotonic in j
-      if (nrun == kRun && xi + floor_small(fminf(xf, xe) - spanf) + 1 >= 0 &&
-          xi + floor_small(fmaxf(xf, xe) - spanf) + 3 <= ncol - 1) {
+      // a full run whose candidate pixels all lie inside the line: no bounds
+      // logic, and only the last weight can need its clamp at zero.  The first
+      // and the last step's t, formed as the loop forms them (t is monotonic in
+      // j), bound every index: rounded another way they may miss by a pixel.
+      const float xs = xf - spanf, te = fmaf((float)(kRun - 1), rf, xs);
+      if (nrun == kRun && xi + floor_small(fminf(xs, te)) + 1 >= 0 &&
+          xi + floor_small(fmaxf(xs, te)) + 3 <= ncol - 1) {
         const float *base = line + xi - 0x4B400000ll + 1;
-        const float xs = xf - spanf;
         float run2 = 0.0f, run3 = 0.0f;
 #pragma unroll 8
         for (int j = 0; j < kRun; ++j, base += rs) {
