@@ -17,7 +17,7 @@ CASES = [(0.7553517346258771, 142.6171879066859, 151, 252),
          (0.6972972450338121, 142.9911856614644, 186, 216),
          (0.6972972450338121, 143.10851924909855, 163, 252),
          (0.6616862921639072, 143.07806922120255, 170, 252),
-         (0.6784457776456341, 142.79022525051575, 189, 216),
+         (0.6784457776456341, 142.7902247737047, 189, 216),
          (-0.43459620383329917, 143.33163676016486, 72, 252),
          (-0.3190045807988174, 142.74986978222145, 39, 216),
          (-0.3299277979919403, 143.17511563920868, 41, 216)]
