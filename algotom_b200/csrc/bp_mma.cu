@@ -97,6 +97,7 @@ constexpr unsigned kInfBits = 0x7f800000u;
 constexpr int kNowhere = 11 << kFrac;     // a position whose weights are both zero
 
 __device__ int g_mma_status;  // bit 0: a CTA gave up waiting
+constexpr unsigned long long kWaitLimit = 1000000000ull;  // ns: about a second, against microseconds in normal operation
 
 struct MmaArgs {
   const unsigned *maxbits;  // [S] largest |sample| of each slice, as bits
@@ -109,6 +110,8 @@ struct MmaArgs {
   float *out;
   long long ors, oss;
   double interior;  // >= 0: only the blocks of bp_interior (centre groups)
+  int inject;       // test only: CTA (0, 0) arms its first copies for 16 bytes
+                    // more than they deliver
 };
 
 // parameters of one (angle, tile)
@@ -130,6 +133,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ bool mbar_test(uint64_t *bar, unsigned parity) {
   unsigned done;
   asm volatile(
@@ -141,15 +147,18 @@ __device__ __forceinline__ bool mbar_test(uint64_t *bar, unsigned parity) {
       : "memory");
   return done != 0;
 }
-// waits for the phase of the given parity; gives up after about a second, or
-// at once when another thread of the CTA has (*bad)
+// Waits for the phase of the given parity; gives up after kWaitLimit, or at once
+// when another thread of the CTA has (*bad).  Then nothing more is requested, the
+// other warps walk on to the end without waiting, over parameters that keep every
+// access inside its buffer whatever has arrived, and no pixel is written.  (With
+// a vote and a way out of the loop after each wait the kernel takes 8-12 % longer.)
 __device__ __forceinline__ void mbar_wait(uint64_t *bar, unsigned parity, volatile int *bad) {
   unsigned long long t0 = 0, t;
   for (int n = 1; !mbar_test(bar, parity); ++n) {
     if (n & 63) continue;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     if (t0 == 0) t0 = t;
-    if (*bad || t - t0 > 1000000000ull) {
+    if (*bad || t - t0 > kWaitLimit) {
       *bad = 1;
       return;
     }
@@ -382,6 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
       mbar_init(&ddone[q], 1);
       mbar_init(&dfree[q], 2);  // the two warps of the high rows
     }
+    if (a.inject && blockIdx.x == 0 && blockIdx.y == 0) mbar_expect_tx(&full[0], 16u);
     bad_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -389,6 +399,12 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
     sel.w03[tid] = make_uint4(select_bytes(tid, 0), select_bytes(tid, 1), select_bytes(tid, 2), select_bytes(tid, 3));
     sel.w45[tid] = make_uint4(select_bytes(tid, 4), select_bytes(tid, 5), 0u, 0u);
   }
+  // parameters that no chunk has written yet: no weights, a window inside the ring
+  if (tid < kRing * kChunk * 4) {
+    prm[tid] = {kNowhere, 0, 0, (int)(smem_u32(smem) >> 4)};
+    edge[tid] = {0, 0};
+  }
+  if (tid < kRing) checked_s[tid] = 0u;
   if (warp == kProducers) {
     asm volatile(
         "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n\t"
@@ -410,7 +426,11 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
     const int ai = lane >> 2;
     for (int k = warp - kProducers - 1; warp > kProducers && k < nchunk; k += 3) {
       const int r = k % kRing;
-      if (k >= kRing) mbar_wait(&empty[r], (unsigned)((k / kRing - 1) & 1), bad);
+      if (k >= kRing) {
+        mbar_wait(&empty[r], (unsigned)((k / kRing - 1) & 1), bad);
+        // (full[r] may still be short of bytes: another arrival would fault)
+        if (__any_sync(0xffffffffu, *bad)) break;
+      }
       unsigned char *dst = smem + (size_t)(r * kChunk + ai) * K::kAngleBytes;
       const int e = r * kChunk * 4 + lane;
       const int rlo = angle_params(a, k * kChunk + ai, x0, y0, lane & 3, smem_u32(dst), prm[e], edge[e]);
@@ -512,7 +532,7 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
         fold(t0 + 2, sum[1], comp[1]);
       }
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");  // every MMA is done
+    asm volatile("bar.sync 1, 128;" ::: "memory");  // every MMA is done (or given up)
     fence_after();
     // totals to the ring, which nothing reads any more:
     // [high sums, the rest of them, low][pixel of 4 tiles][S + 1]
@@ -554,11 +574,15 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
     const __half2 minus = __halves2half2(__float2half_rn(high ? -1024.f : -2048.f), __float2half_rn(-1024.f));
     const uint32_t wcol = tmem + ((uint32_t)((row >> 5) * 32) << 16) + 256u + (uint32_t)(quad * 2 * 8 * kStep);
 
-    // the weights of kStep angles from ring entry e (angle i of the launch)
+    // The weights of kStep angles from ring entry e (angle i of the launch).  How
+    // these loops lie in the instruction cache, which 28 warps share, matters: with
+    // the rarer checked form rolled up and a chunk's two steps unrolled, 901 x 1280
+    // takes 5.38 (16 slices), 6.01 (24) and 6.36 ms (32); both forms unrolled and
+    // the steps rolled up, 5.93, 6.47 and 6.76.
     auto weights = [&](auto checked_tag, int e, int i, uint32_t col) {
       constexpr bool kChecked = decltype(checked_tag)::value;
       const TilePrm *pp = prm + e * 4 + quad;
-#pragma unroll
+#pragma unroll (kChecked ? 1 : 2)
       for (int u2 = 0; u2 < kStep; u2 += 2) {
         uint32_t w[16];
 #pragma unroll
@@ -575,7 +599,7 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
                 if (abs(q - ed.qlo) < kTol || abs(q - ed.qmax) < kTol) {
                   // the reference's expression and rounding order in FP64
                   const double ic = 0.5 * (double)(ncol - 1);
-                  const double2 cs = a.trig[i + u2 + u];
+                  const double2 cs = a.trig[min(i + u2 + u, a.nrow - 1)];  // (past it only after a wait gave up)
                   const double xq = x0 + (quad & 1) * kTile + tx, yq = y0 + (quad >> 1) * kTile + ty;
                   const double pe =
                       __dadd_rn(__dadd_rn(__dmul_rn(xq - ic, cs.x), __dmul_rn(yq - ic, cs.y)), a.center);
@@ -606,7 +630,7 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
       const int r = k % kRing;
       mbar_wait(&full[r], (unsigned)((k / kRing) & 1), bad);
       const bool chk = (checked_s[r] >> quad) & 1u;
-#pragma unroll 1
+#pragma unroll
       for (int st = 0; st < kChunk / kStep; ++st, ++step) {
         const int slot = step & 1;
         // the MMAs that read this slot two steps ago are done
@@ -626,9 +650,9 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
   __syncthreads();
   if (*bad) {
     if (tid == 0) atomicOr(&g_mma_status, 1);
-    // copies and MMAs that are still in flight end in microseconds; this CTA's
-    // memory is its own for another millisecond
-    for (int n = 0; n < 64; ++n) __nanosleep(16000);
+    // this CTA's memory stays its own until what is in flight has ended: copies
+    // and MMAs, at worst all of them (128 clocks an angle)
+    for (int n = 0; n < 64 + a.nrow / 128; ++n) __nanosleep(16000);
     __syncthreads();
   }
   if (!*bad && tid < 3 * kRegion * kRegion) {
@@ -846,7 +870,7 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
                                      double center, int edge_pad, double mask_r2, float scale, float *out,
                                      int64_t out_row_stride, int64_t out_slice_stride, int flags, void *workspace,
                                      int64_t workspace_bytes, void *stream) {
-  if (flags & ~16) return atb::fail(ATB_EINVAL, "atb_backproject_stack: unknown flags %d", flags);
+  if (flags & ~48) return atb::fail(ATB_EINVAL, "atb_backproject_stack: unknown flags %d", flags);
   cudaStream_t st = atb::as_stream(stream);
   const int64_t need = atb_backproject_stack_workspace(sino_dtype, nrow, nslice, ncol);
   const int esize = sino_dtype == ATB_F32 ? 4 : 2;
@@ -868,13 +892,14 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
       a.trig = reinterpret_cast<const double2 *>(trig);
       a.nrow = nrow; a.ncol = ncol; a.nsl = n;
       a.center = center; a.edge_pad = edge_pad ? 1 : 0; a.mask_r2 = mask_r2; a.scale = scale;
-            a.out = dst; a.ors = out_row_stride; a.oss = out_slice_stride;
+      a.out = dst; a.ors = out_row_stride; a.oss = out_slice_stride;
       a.interior = -1.0;
+      a.inject = (flags >> 5) & 1;
       rc = launch(a, S, static_cast<unsigned char *>(workspace) + kHeader, st);
       if (rc != ATB_OK) return rc;
       // runs only where a sample is not finite
       rc = atb::bp_gather(src, sino_dtype, sino_row_stride, sino_slice_stride, nrow, n, ncol, trig, center, edge_pad,
-                          mask_r2, scale, dst, out_row_stride, out_slice_stride, flags, a.maxbits, nullptr, stream);
+                          mask_r2, scale, dst, out_row_stride, out_slice_stride, flags & 16, a.maxbits, nullptr, stream);
       if (rc != ATB_OK) return rc;
     }
     if (first == nslice) return ATB_OK;
@@ -926,6 +951,7 @@ extern "C" int atb_backproject_centers_stack(const float *sino, int64_t sino_row
       a.out = out + (int64_t)first * out_center_stride; a.ors = out_row_stride; a.oss = out_center_stride;
       const double reach = (c0 < (double)(ncol - 1) - c1 ? c0 : (double)(ncol - 1) - c1) - 1e-2;
       a.interior = reach > 0.0 ? reach : 0.0;
+      a.inject = 0;
       rc = launch(a, S, packed, st);
       if (rc != ATB_OK) return rc;
       // the blocks whose positions reach an edge of the detector for some

@@ -223,7 +223,9 @@ int atb_backproject(const void *sino, int sino_dtype, int64_t sino_row_stride,
  * more CTAs and add the parts in FP64.  Everything else, and every call
  * without a (large enough) workspace, is atb_backproject.
  *
- *   flags      bit 4 as atb_backproject (the same results), else 0
+ *   flags      bit 4 as atb_backproject (the same results); bit 5 (tests only):
+ *              the first CTA's first copies are armed for 16 bytes more than
+ *              they deliver, and it gives up; else 0
  *   workspace  128-byte aligned device scratch of
  *              atb_backproject_stack_workspace bytes (0: none is used), free
  *              for reuse when the call's work on the stream is done
@@ -290,8 +292,9 @@ int atb_backproject_centers_stack(const float *sino, int64_t sino_row_stride,
 
 /*
  * Status word of the back-projection kernels: bit 0 is set when a CTA gave
- * up waiting (after about 70 ms) for a TMA window load and left its tile
- * unwritten.  Returns the word (0 = no such event since the last reset) and
+ * up waiting and left its tile unwritten: a gather CTA after about 70 ms for
+ * a TMA window load, a tensor-core CTA after about a second for a load, its
+ * weights or its sums.  Returns the word (0 = no such event since the last reset) and
  * clears it when reset != 0; negative on a CUDA error.  Synchronises with
  * the device.
  */
