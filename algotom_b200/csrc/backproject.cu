@@ -118,8 +118,8 @@ struct BPArgs {
   int wait_polls;  // polls before a staging wait gives up (kWaitPolls)
   int inject;      // test only: CTA (0, 0, 0) arms its first staging wait
                    // for 16 bytes more than its copies deliver
-  const unsigned *gate;  // null, or ngate words (float bits): do nothing unless
-  int ngate;             // one of them is not finite
+  const unsigned *gate;  // null, or a gate for ngate slices: do nothing unless
+  int ngate;             // bp_left_to_gather
   // angle groups: CTA layer g of ngroup walks the angles from g * group_rows
   // and leaves its compensated totals, not pixels, in part
   // [ngroup][nslice][ncol][ncol] (total, compensation)
@@ -879,8 +879,8 @@ __global__ void __launch_bounds__(BPCfg<T, S, V>::kThreads, BPCfg<T, S, V>::kMin
   using K = BPCfg<T, S, V>;
   extern __shared__ __align__(16) unsigned char smem[];
   if (a.gate) {
-    const bool finite = !__syncthreads_or((int)threadIdx.x < a.ngate && a.gate[threadIdx.x] >= 0x7f800000u);
-    if (finite && (a.interior < 0.0 || atb::bp_interior(blockIdx.x * K::TX, blockIdx.y * K::TY, a.ncol, a.interior)))
+    const bool left = atb::bp_left_to_gather(a.gate, a.ngate, a.nrow);
+    if (!left && (a.interior < 0.0 || atb::bp_interior(blockIdx.x * K::TX, blockIdx.y * K::TY, a.ncol, a.interior)))
       return;
   }
   int bz = blockIdx.z;

@@ -13,14 +13,14 @@
 // the number of slices; here the weights of a pixel are formed once and
 // serve up to 32 slices.
 //
-// Precision.  Both factors are split in two float16 terms, so that no
-// product loses what FP32 would keep:
+// Precision.  Both factors are split in two float16 terms:
 // - positions are 32-bit fixed point (2^-26 bins) from an FP64 origin per
 //   (tile, angle), their fraction rounded to 20 bits: 10 for the high weight
 //   (integers 1024 - u and u in units of 2^-10) and 10 for the low one
 //   (-v, v in units of 2^-20); the weights are exact in float16 and sum to 1;
-// - samples, scaled per slice by a power of two to below 2^15, are
-//   hi + lo float16 (22 bits).
+// - samples, scaled per slice by a power of two to below 2^15, are hi + lo
+//   float16: 22 bits down to 2^-17 of the slice's largest sample, and a fixed
+//   2^-40 of that sample below.
 // The accumulator tile has 128 rows, 64 pixels x (high, low weight), and 2 S
 // columns, S slices x (hi, lo): all four partial products.  The tensor cores
 // add in FP32 with truncation (measured: a relative bias of 5e-8 over 8
@@ -31,9 +31,10 @@
 // Error against FP64 at 901 x 1024: 1.4e-7 (2.3e-7 with the gather kernel,
 // whose positions carry 1e-5 bins of FP32 rounding).
 //
-// A stack that holds a non-finite sample is left to the gather kernel (0
-// times an infinity must stay out of the pixels that do not read it): the
-// scan for the slices' largest magnitudes sees it, this kernel's CTAs leave
+// A stack that holds a non-finite sample (0 times an infinity must stay out of
+// the pixels that do not read it), or so faint ones beside its largest that 2^-40
+// of that shows, is left to the gather kernel: the scan for the slices' largest
+// magnitudes and the packing see it (bp_left_to_gather), this kernel's CTAs leave
 // at once and the gather kernel's CTAs, launched behind a gate, run.
 //
 // One CTA (one per SM) owns 16 x 16 pixels, four tiles, and walks the angles in
@@ -92,8 +93,8 @@ constexpr int kThreads = 28 * 32;
 constexpr int kRegsWeights = 64, kRegsTotals = 168, kRegsHelpers = 40;
 constexpr int kFrac = 26;                 // fraction bits of a position
 constexpr float kTolBins = 2e-3f;         // as the gather kernel's edge decision
-constexpr int kHeader = 256;              // workspace bytes before the packed samples
-constexpr unsigned kInfBits = 0x7f800000u;
+constexpr int kHeader = 512;              // workspace bytes before the packed samples: the gate's words
+static_assert(atb::kGateWords * sizeof(unsigned) <= kHeader, "the gate fits its header");
 constexpr int kNowhere = 11 << kFrac;     // a position whose weights are both zero
 
 __device__ int g_mma_status;  // bit 0: a CTA gave up waiting
@@ -101,6 +102,8 @@ constexpr unsigned long long kWaitLimit = 1000000000ull;  // ns: about a second,
 
 struct MmaArgs {
   const unsigned *maxbits;  // [S] largest |sample| of each slice, as bits
+  const unsigned *gate;     // bp_left_to_gather, for ngate slices
+  int ngate;
   const double2 *trig;
   int nrow, ncol, nsl;  // nsl: live slices (<= S)
   double center;
@@ -362,8 +365,7 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int x0 = blockIdx.x * kRegion, y0 = blockIdx.y * kRegion;
   const int ncol = a.ncol, cm = ncol / 2;
-  // non-finite samples: the gather kernel takes the stack
-  if (__syncthreads_or(tid < S && a.maxbits[tid] >= kInfBits)) return;
+  if (atb::bp_left_to_gather(a.gate, a.ngate, a.nrow)) return;
   if (a.interior >= 0.0 && !atb::bp_interior(x0, y0, ncol, a.interior)) return;
   // a region wholly outside the circle mask is zero
   if (a.mask_r2 >= 0.0) {
@@ -684,18 +686,32 @@ __global__ void __launch_bounds__(kThreads, 1) bp_mma_kernel(MmaArgs a, const __
   }
 }
 
+// Adds a warp's faint pairs (a sample and the one before it, both scaled) to
+// *pairs.  Every lane calls it.
+__device__ __forceinline__ void count_faint(float v, float before, bool valid, unsigned *pairs) {
+  const unsigned n = __popc(__ballot_sync(
+      0xffffffffu, valid && fabsf(v) < atb::kFaint && fabsf(before) < atb::kFaint && (v != 0.f || before != 0.f)));
+  if (n > 0u && (threadIdx.x & 31) == 0) atomicAdd(pairs, n);
+}
+
 // The S "slices" of a centre group: slice m is the one row of each angle, read m
 // spacing bins further on.  One word of maxbits serves them all (the others
-// repeat it).
+// repeat it).  count: the first group of a call, which counts the row's faint
+// pairs.
 __global__ void __launch_bounds__(256) pack_centers_kernel(const float *sino, long long srs, int ncol, int nsl, int S,
-                                                           int spacing, unsigned *maxbits, uint4 *dst) {
+                                                           int spacing, bool count, unsigned *maxbits, uint4 *dst) {
   const int i = blockIdx.y, g = blockIdx.z;
   const unsigned bits = maxbits[0];
   if (i == 0 && blockIdx.x == 0 && threadIdx.x < 8) maxbits[S + 8 * g + threadIdx.x] = bits;
   const float sc = __int_as_float((atb::bp_sample_exponent(bits) + 127) << 23);
   const float *row = sino + i * srs;
   uint4 *hi = dst + ((long long)i * (S / 4) + g) * ncol, *lo = hi + (long long)(S / 8) * ncol;
-  for (int d = blockIdx.x * 256 + threadIdx.x; d < ncol; d += gridDim.x * 256) {
+  const int d = blockIdx.x * 256 + threadIdx.x;
+  if (count && g == 0) {
+    const float v = d < ncol ? __ldg(row + d) * sc : 0.f, before = d > 0 && d < ncol ? __ldg(row + d - 1) * sc : v;
+    count_faint(v, before, d > 0 && d < ncol, maxbits + atb::kGatePairs);
+  }
+  if (d < ncol) {
     unsigned h[4], l[4];
 #pragma unroll
     for (int u = 0; u < 8; u += 2) {
@@ -732,32 +748,38 @@ __global__ void __launch_bounds__(256) absmax_kernel(const T *sino, long long sr
 }
 
 // [angle][slice][bin] samples -> [angle][G][bin][8] float16, groups of 8
-// slices: first the hi parts of all S slices, then the lo parts.
+// slices: first the hi parts of all S slices, then the lo parts.  Counts the
+// slices' faint pairs (of 16-bit samples, which one term holds, too).
 template <typename T>
 __global__ void __launch_bounds__(256) pack_kernel(const T *sino, long long srs, long long sss, int nrow, int ncol,
-                                                   int nsl, int S, const unsigned *maxbits, uint4 *dst) {
-  const int i = blockIdx.y, g = blockIdx.z;
-  float sc[8];
-#pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const int k = 8 * g + u;
-    sc[u] = k < nsl ? __int_as_float((atb::bp_sample_exponent(maxbits[k]) + 127) << 23) : 0.f;
-  }
+                                                   int nsl, int S, unsigned *gate, uint4 *dst) {
+  const int i = blockIdx.y, g = blockIdx.z, lane = threadIdx.x & 31;
   const T *row = sino + i * srs + 8 * g * sss;
   uint4 *hi = dst + ((long long)i * (S / 4) + g) * ncol, *lo = hi + (long long)(S / 8) * ncol;
-  for (int d = blockIdx.x * 256 + threadIdx.x; d < ncol; d += gridDim.x * 256) {
-    unsigned h[4], l[4];
+  const int d = blockIdx.x * 256 + threadIdx.x;
+  unsigned h[4], l[4];
 #pragma unroll
-    for (int u = 0; u < 8; u += 2) {
-      float v[2];
+  for (int u = 0; u < 8; u += 2) {
+    float v[2];
 #pragma unroll
-      for (int t = 0; t < 2; ++t) v[t] = 8 * g + u + t < nsl ? atb::load_as_float(row + (u + t) * sss + d) * sc[u + t] : 0.f;
-      const __half2 hh = __floats2half2_rn(v[0], v[1]);
-      const float2 hf = __half22float2(hh);
-      const __half2 ll = __floats2half2_rn(v[0] - hf.x, v[1] - hf.y);
-      h[u / 2] = *reinterpret_cast<const unsigned *>(&hh);
-      l[u / 2] = *reinterpret_cast<const unsigned *>(&ll);
+    for (int t = 0; t < 2; ++t) {
+      const int k = 8 * g + u + t;
+      v[t] = 0.f;
+      if (k >= nsl) continue;
+      const float sc = __int_as_float((atb::bp_sample_exponent(gate[k]) + 127) << 23);
+      const T *p = row + (u + t) * sss;
+      if (d < ncol) v[t] = atb::load_as_float(p + d) * sc;
+      float before = __shfl_up_sync(0xffffffffu, v[t], 1);
+      if (lane == 0 && d > 0 && d < ncol) before = atb::load_as_float(p + d - 1) * sc;
+      count_faint(v[t], before, d > 0 && d < ncol, gate + atb::kGatePairs + k);
     }
+    const __half2 hh = __floats2half2_rn(v[0], v[1]);
+    const float2 hf = __half22float2(hh);
+    const __half2 ll = __floats2half2_rn(v[0] - hf.x, v[1] - hf.y);
+    h[u / 2] = *reinterpret_cast<const unsigned *>(&hh);
+    l[u / 2] = *reinterpret_cast<const unsigned *>(&ll);
+  }
+  if (d < ncol) {
     hi[d] = make_uint4(h[0], h[1], h[2], h[3]);
     lo[d] = make_uint4(l[0], l[1], l[2], l[3]);
   }
@@ -888,7 +910,8 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
                    : prepare<__half>(src, sino_row_stride, sino_slice_stride, nrow, n, ncol, S, workspace, st);
       if (rc != ATB_OK) return rc;
       MmaArgs a;
-      a.maxbits = static_cast<const unsigned *>(workspace);
+      a.maxbits = a.gate = static_cast<const unsigned *>(workspace);
+      a.ngate = n;
       a.trig = reinterpret_cast<const double2 *>(trig);
       a.nrow = nrow; a.ncol = ncol; a.nsl = n;
       a.center = center; a.edge_pad = edge_pad ? 1 : 0; a.mask_r2 = mask_r2; a.scale = scale;
@@ -897,9 +920,9 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
       a.inject = (flags >> 5) & 1;
       rc = launch(a, S, static_cast<unsigned char *>(workspace) + kHeader, st);
       if (rc != ATB_OK) return rc;
-      // runs only where a sample is not finite
+      // runs only where bp_left_to_gather
       rc = atb::bp_gather(src, sino_dtype, sino_row_stride, sino_slice_stride, nrow, n, ncol, trig, center, edge_pad,
-                          mask_r2, scale, dst, out_row_stride, out_slice_stride, flags & 16, a.maxbits, nullptr, stream);
+                          mask_r2, scale, dst, out_row_stride, out_slice_stride, flags & 16, a.gate, nullptr, stream);
       if (rc != ATB_OK) return rc;
     }
     if (first == nslice) return ATB_OK;
@@ -940,11 +963,13 @@ extern "C" int atb_backproject_centers_stack(const float *sino, int64_t sino_row
       const double c0 = center + (double)first * (double)spacing, c1 = c0 + (double)(n - 1) * (double)spacing;
       // samples of the first centre's frame: later centres read further on
       pack_centers_kernel<<<dim3((ncol + 255) / 256, nrow, S / 8), 256, 0, st>>>(sino, sino_row_stride, ncol, n, S,
-                                                                                spacing, maxbits, packed);
+                                                                                spacing, first == 0, maxbits, packed);
       rc = atb::check_launch("atb_backproject_centers_stack (pack)");
       if (rc != ATB_OK) return rc;
       MmaArgs a;
       a.maxbits = maxbits + S;
+      a.gate = maxbits;
+      a.ngate = 1;
       a.trig = reinterpret_cast<const double2 *>(trig);
       a.nrow = nrow; a.ncol = ncol; a.nsl = n;
       a.center = c0; a.edge_pad = edge_pad ? 1 : 0; a.mask_r2 = mask_r2; a.scale = scale;
@@ -957,7 +982,7 @@ extern "C" int atb_backproject_centers_stack(const float *sino, int64_t sino_row
       // the blocks whose positions reach an edge of the detector for some
       // centre: each centre has its own edges there
       rc = atb::bp_gather_centers(sino, sino_row_stride, nrow, ncol, trig, c0, spacing, n, edge_pad, mask_r2, scale,
-                                  a.out, out_row_stride, out_center_stride, flags, maxbits, 1, a.interior, stream);
+                                  a.out, out_row_stride, out_center_stride, flags, a.gate, a.ngate, a.interior, stream);
       if (rc != ATB_OK) return rc;
     }
     if (first == ncenter) return ATB_OK;

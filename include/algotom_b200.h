@@ -217,11 +217,14 @@ int atb_backproject(const void *sino, int sino_dtype, int64_t sino_row_stride,
  * atb_backproject, given a workspace.  Stacks of 15 and more
  * float32 or float16 slices run on the tensor cores, up to 32 slices per
  * launch: samples and weights are split in two float16 terms each and the sums
- * are compensated FP32, so that results differ from atb_backproject's by
- * rounding only; stacks with non-finite samples give atb_backproject's
- * results.  Launches whose tiles do not fill the GPU split the angles over
- * more CTAs and add the parts in FP64.  Everything else, and every call
- * without a (large enough) workspace, is atb_backproject.
+ * are compensated FP32.  A sample is held to 22 bits down to 2^-17 of its
+ * slice's largest, so that results differ from atb_backproject's by rounding
+ * only.  Where a slice holds more pairs of neighbouring samples below about
+ * 2^-16 of its largest (zeros apart) than a sixteenth of its angles, or a sample
+ * is not finite, its launch's slices are atb_backproject's.  Launches whose
+ * tiles do not fill the GPU split the angles over more CTAs and add the parts in
+ * FP64.  Everything else, and every call without a (large enough) workspace, is
+ * atb_backproject.
  *
  *   flags      bit 4 as atb_backproject (the same results); bit 5 (tests only):
  *              the first CTA's first copies are armed for 16 bytes more than
@@ -273,7 +276,8 @@ int atb_backproject_centers(const float *sino, int64_t sino_row_stride,
 /*
  * atb_backproject_centers, given a workspace: groups of 15 and more centres run
  * on the tensor cores (up to 32 per launch) where no position leaves the
- * detector for any of them, the rest of the image and every call without a
+ * detector for any of them, the rest of the image, sinograms of the kind that
+ * atb_backproject_stack leaves to atb_backproject, and every call without a
  * (large enough) workspace as atb_backproject_centers does.  Results differ by
  * rounding only.
  *
