@@ -25,8 +25,8 @@
 // columns, S slices x (hi, lo): all four partial products.  The tensor cores
 // add in FP32 with truncation (measured: a relative bias of 5e-8 over 8
 // additions, 1.3e-7 over 16, 2.5e-5 over 1024), so the sums leave TMEM every 16
-// angles (8 with edge padding) and are added with Kahan compensation in
-// registers; the other three products, below 2^-10 of the high terms' one, stay
+// angles (8 with edge padding and where the angles are many for the image) and are
+// added with Kahan compensation in registers; the other three products, below 2^-10 of the high terms' one, stay
 // in TMEM to the end.  A pixel is rounded once, after the small terms joined.
 // Error against FP64 at 901 x 1024: 1.4e-7 (2.3e-7 with the gather kernel,
 // whose positions carry 1e-5 bins of FP32 rounding).
@@ -76,12 +76,8 @@ constexpr int kBins = 28;                 // bins staged per angle: 12 (the larg
 constexpr int kChunk = 8;                 // angles per chunk
 constexpr int kRing = 4;                  // chunks in flight
 constexpr int kStep = 4;                  // angles per weight slot
-// Steps between two reads of an accumulator: 16 angles, and 8 with edge padding
-// (BPF), whose samples of one sign add the truncations up and whose 2-D ramp
-// filter then magnifies them.  BPF error against FP64 at 901 x 1280 with 4, 8
-// and 16 angles: 3.95e-6, 3.95e-6, 4.08e-6 (4.23e-6 with the gather kernel), in
-// 10.6, 10.1 and 10.0 ms.
-constexpr int kFoldPlain = 4, kFoldEdge = 2;
+// Steps between two reads of an accumulator: 16 angles, or 8 (fold_steps)
+constexpr int kFoldLong = 4, kFoldShort = 2;
 // warps 0-15 form the weights (four for each tile), 16-19 keep the totals,
 // 20-23 issue a tile's MMAs each, 25-27 stage (every third chunk each: one warp
 // alone, waiting for its FP64 results, takes 2.29 ms at 361 x 1024 with 32
@@ -821,14 +817,31 @@ int launch_mma(const MmaArgs &a, void *packed, cudaStream_t st) {
   return atb::check_launch("atb_backproject_stack");
 }
 
+// Steps between two reads of an accumulator.  The truncations add up to a bias,
+// the same for every pixel, that the angles do not average out: after 16 angles
+// 1.4e-7 of an image, after 8 0.7e-7 (half of it at 200 pixels).  The gather
+// kernel's error, from its positions, falls as the angles and grows with the
+// image, 2.2e-7 (ncol / 1024) sqrt(901 / nrow), so that 16 angles are the less
+// exact choice from nrow = ncol^2 / 1100 on.  Errors of filtered sinograms
+// against FP64 with 16 angles, with 8, and with the gather kernel (1e-8):
+//   901 x 200: 10.1, 3.8, 6.5;  901 x 512: 13.6, 6.2, 12.0;  901 x 1024: 14.1,
+//   7.8, 22.5;  1801 x 320: 11.8, 4.9, 6.2;  1801 x 720: 13.8, 6.5, 11.6
+// 8 angles cost 1801 x 2560 with 32 slices 59.4 ms instead of 55.7.  With edge
+// padding (BPF) the samples have one sign, so that the bias is the larger, and the
+// 2-D ramp filter magnifies it: BPF of 901 x 1280 has 4.0e-6 with 8 and 4.1e-6
+// with 16 angles (4.2e-6 with the gather kernel).
+int fold_steps(const MmaArgs &a) {
+  return a.edge_pad || (long long)a.ncol * a.ncol < 600ll * a.nrow ? kFoldShort : kFoldLong;
+}
+
 int launch(const MmaArgs &a, int S, void *packed, cudaStream_t st) {
-  if (a.edge_pad)
-    return S == 16   ? launch_mma<16, kFoldEdge>(a, packed, st)
-           : S == 24 ? launch_mma<24, kFoldEdge>(a, packed, st)
-                     : launch_mma<32, kFoldEdge>(a, packed, st);
-  return S == 16   ? launch_mma<16, kFoldPlain>(a, packed, st)
-         : S == 24 ? launch_mma<24, kFoldPlain>(a, packed, st)
-                   : launch_mma<32, kFoldPlain>(a, packed, st);
+  if (fold_steps(a) == kFoldShort)
+    return S == 16   ? launch_mma<16, kFoldShort>(a, packed, st)
+           : S == 24 ? launch_mma<24, kFoldShort>(a, packed, st)
+                     : launch_mma<32, kFoldShort>(a, packed, st);
+  return S == 16   ? launch_mma<16, kFoldLong>(a, packed, st)
+         : S == 24 ? launch_mma<24, kFoldLong>(a, packed, st)
+                   : launch_mma<32, kFoldLong>(a, packed, st);
 }
 
 template <typename T>
@@ -853,9 +866,13 @@ int prepare(const void *sino, long long srs, long long sss, int nrow, int nsl, i
 // slices, at 901 x 1280 6.1 ms, and the gather kernel 0.43 ms per slice: 6.0
 // for 14, 6.5 for 15.  bfloat16 samples stay with the gather kernel, whose
 // interpolation differences are bfloat16 too: a user's results would move by
-// that rounding (2e-4) for a faster kernel.
-int next_group(int sino_dtype, int n) {
-  if (sino_dtype == ATB_BF16) return 0;
+// that rounding (2e-4) for a faster kernel.  So do stacks of more angles than the
+// truncations bear, whose sums the gather kernel, averaging over its positions'
+// errors, holds the better (1e-8, 8 angles between two reads, and gather): 7201 x
+// 320: 4.7, 3.8; x 512: 5.8, 4.9; 30001 x 200: 4.4, 2.7 (the small products, which
+// stay in TMEM to the end, then show).
+int next_group(int sino_dtype, int nrow, int ncol, int n) {
+  if (sino_dtype == ATB_BF16 || nrow > 8192 || (nrow > 2048 && (long long)ncol * ncol < 120ll * nrow)) return 0;
   if (n >= 32) return 32;
   return n >= 15 ? n : 0;
 }
@@ -877,12 +894,12 @@ int bp_mma_status(int reset) {
 
 extern "C" int64_t atb_backproject_stack_workspace(int sino_dtype, int nrow, int nslice, int ncol) {
   if (nrow < 1 || nslice < 1 || ncol < 1 || nrow > 65535 || ncol > (1 << 16)) return 0;
-  const int n = next_group(sino_dtype, nslice);
+  const int n = next_group(sino_dtype, nrow, ncol, nslice);
   const int64_t packed = n ? kHeader + (int64_t)nrow * ncol * padded(n) * 4 : 0;
   // slices left over after the last launch of the tensor cores
   int left = nslice;
   if (n == 32) left %= 32;
-  if (next_group(sino_dtype, left)) left = 0;
+  if (next_group(sino_dtype, nrow, ncol, left)) left = 0;
   const int64_t split = left ? atb::bp_gather_workspace(nrow, left, ncol) : 0;
   return packed > split ? packed : split;
 }
@@ -901,7 +918,7 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
   const bool args_ok = sino && trig && out && (sino_dtype == ATB_F32 || sino_dtype == ATB_F16 || sino_dtype == ATB_BF16) &&
                        center >= 0.0 && center < (double)ncol;
   if (args_ok && work_ok) {
-    for (int n; (n = next_group(sino_dtype, nslice - first)) > 0; first += n) {
+    for (int n; (n = next_group(sino_dtype, nrow, ncol, nslice - first)) > 0; first += n) {
       const int S = padded(n);
       const char *src = static_cast<const char *>(sino) + (int64_t)first * sino_slice_stride * esize;
       float *dst = out + (int64_t)first * out_slice_stride;
@@ -935,7 +952,7 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
 
 extern "C" int64_t atb_backproject_centers_workspace(int nrow, int ncol, int ncenter) {
   if (nrow < 1 || ncol < 1 || ncenter < 1 || nrow > 65535 || ncol > (1 << 16)) return 0;
-  const int n = next_group(ATB_F32, ncenter);
+  const int n = next_group(ATB_F32, nrow, ncol, ncenter);
   return n ? kHeader + (int64_t)nrow * ncol * padded(n) * 4 : 0;
 }
 
@@ -958,7 +975,7 @@ extern "C" int atb_backproject_centers_stack(const float *sino, int64_t sino_row
     absmax_kernel<float><<<dim3(nrow < 256 ? nrow : 256, 1), 256, 0, st>>>(sino, sino_row_stride, 0, nrow, ncol, maxbits);
     int rc = atb::check_launch("atb_backproject_centers_stack (scan)");
     if (rc != ATB_OK) return rc;
-    for (int n; (n = next_group(ATB_F32, ncenter - first)) > 0; first += n) {
+    for (int n; (n = next_group(ATB_F32, nrow, ncol, ncenter - first)) > 0; first += n) {
       const int S = padded(n);
       const double c0 = center + (double)first * (double)spacing, c1 = c0 + (double)(n - 1) * (double)spacing;
       // samples of the first centre's frame: later centres read further on
