@@ -878,6 +878,40 @@ int next_group(int sino_dtype, int nrow, int ncol, int n) {
 }
 int padded(int n) { return (n + 7) / 8 * 8; }
 
+// Angles from which a group of n slices is worth its scan, packing and launch
+// (the gather kernel has one launch, of a cost per slice).  Time against the
+// gather kernel's by angles, read off 15 to 32 slices of 32 to 2560 pixels:
+//   up to 160 pixels  16 slices: 1.15 (16), 0.85 (24); 32 slices: 1.07 (24), 0.96 (32)
+//   24 slices         512: 1.11 (32), 0.95 (48); 1536: 1.08 (48), 0.94 (64)
+//   32                800: 1.06 (24), 1.00 (32), 0.85 (48)
+//   21                1536: 1.03 (64), 0.91 (96); 2560: 1.05 (64), 0.93 (96)
+//   18, 20            1536: 1.03 (96), 0.96 (128); 2560: 1.05 (96), 0.98 (128)
+//   17                800: 1.00 (64); 1536: 1.02 (128), 0.94 (192)
+//   16                320: 1.01 (64); 800: 0.98 (128); 1536: 1.01 (256); 2560: 1.00 (384)
+//   15                800: 0.94 (64); 1536: 0.99 (256); 2560: 1.00 (384): the two more
+//                     launches of the gather kernel's remainder weigh less and less
+int fewest_angles(int n, int ncol) {
+  if (ncol <= 160) return n > 16 ? 32 : 24;
+  if (n >= 18) return n >= 28 ? 48 : n >= 24 ? 56 : n >= 21 ? 72 : 120;
+  const int w = ncol < 1536 ? ncol : 1536;
+  const int by_size = n == 17 ? 168 * w / 1536 : n == 16 ? 320 * w / 1536 : 320 * w / 1536 * w / 1536;
+  return by_size > 24 ? by_size : 24;
+}
+// The same for a group of n centres, whose gather kernel reads one sinogram for
+// all of them and whose ring stays with it.
+//   15  512: 1.06 (16), 0.89 (32); 800: 1.01 (64), 0.89 (128); 1536: 1.06 (128), 0.91 (192)
+//   16  320: 1.26 (512); 700: 0.91 (192), 0.87 (361); 1100: 0.95 (361)
+//   20  200: 1.15 (512); 400: 0.94 (512); 512: 1.02 (96), 0.93 (128)
+//   28  320: 1.02 (512); 400: 0.95 (192); 700: 0.95 (96)
+//   32  200: 1.13 (512); 400: 0.97 (512); 700: 0.92 (96); 1536: 0.79 (96)
+// Without a remainder of 1 to 3 centres the gather kernel has one launch, and
+// small images are mostly ring.
+bool centers_worth(int n, int nrow, int ncol) {
+  if (n % 4) return nrow >= (ncol > 144 ? ncol / 6 : 24);
+  if (n == 16) return nrow >= 256 && ncol >= 640;
+  return nrow >= 128 && ncol >= 400;
+}
+
 }  // namespace
 
 namespace atb {
@@ -909,7 +943,9 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
                                      double center, int edge_pad, double mask_r2, float scale, float *out,
                                      int64_t out_row_stride, int64_t out_slice_stride, int flags, void *workspace,
                                      int64_t workspace_bytes, void *stream) {
-  if (flags & ~48) return atb::fail(ATB_EINVAL, "atb_backproject_stack: unknown flags %d", flags);
+  if (flags & ~112) return atb::fail(ATB_EINVAL, "atb_backproject_stack: unknown flags %d", flags);
+  const bool always = flags & 64;
+  flags &= ~64;
   cudaStream_t st = atb::as_stream(stream);
   const int64_t need = atb_backproject_stack_workspace(sino_dtype, nrow, nslice, ncol);
   const int esize = sino_dtype == ATB_F32 ? 4 : 2;
@@ -919,6 +955,7 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
                        center >= 0.0 && center < (double)ncol;
   if (args_ok && work_ok) {
     for (int n; (n = next_group(sino_dtype, nrow, ncol, nslice - first)) > 0; first += n) {
+      if (!always && nrow < fewest_angles(n, ncol)) break;
       const int S = padded(n);
       const char *src = static_cast<const char *>(sino) + (int64_t)first * sino_slice_stride * esize;
       float *dst = out + (int64_t)first * out_slice_stride;
@@ -944,6 +981,8 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
     }
     if (first == nslice) return ATB_OK;
   }
+  // (the workspace is sized for the angle groups of what next_group leaves)
+  if (work_ok && next_group(sino_dtype, nrow, ncol, nslice - first)) workspace = nullptr;
   return atb::bp_gather(args_ok ? static_cast<const char *>(sino) + (int64_t)first * sino_slice_stride * esize : sino,
                         sino_dtype, sino_row_stride, sino_slice_stride, nrow, nslice - first, ncol, trig, center,
                         edge_pad, mask_r2, scale, out ? out + (int64_t)first * out_slice_stride : out, out_row_stride,
@@ -963,6 +1002,8 @@ extern "C" int atb_backproject_centers_stack(const float *sino, int64_t sino_row
                                              void *workspace, int64_t workspace_bytes, void *stream) {
   cudaStream_t st = atb::as_stream(stream);
   const int64_t need = atb_backproject_centers_workspace(nrow, ncol, ncenter);
+  const bool always = flags & 64;
+  flags &= ~64;
   int first = 0;
   // (arguments that atb_backproject_centers refuses go there)
   if (sino && trig && out && spacing >= 1 && spacing <= 56 && center >= 0.0 &&
@@ -970,14 +1011,21 @@ extern "C" int atb_backproject_centers_stack(const float *sino, int64_t sino_row
       workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 128 == 0) {
     unsigned *maxbits = static_cast<unsigned *>(workspace);
     uint4 *packed = reinterpret_cast<uint4 *>(static_cast<unsigned char *>(workspace) + kHeader);
-    if (cudaMemsetAsync(workspace, 0, kHeader, st) != cudaSuccess)
-      return atb::fail(ATB_ECUDA, "atb_backproject_centers_stack: %s", cudaGetErrorString(cudaGetLastError()));
-    absmax_kernel<float><<<dim3(nrow < 256 ? nrow : 256, 1), 256, 0, st>>>(sino, sino_row_stride, 0, nrow, ncol, maxbits);
-    int rc = atb::check_launch("atb_backproject_centers_stack (scan)");
-    if (rc != ATB_OK) return rc;
+    int rc;
     for (int n; (n = next_group(ATB_F32, nrow, ncol, ncenter - first)) > 0; first += n) {
       const int S = padded(n);
       const double c0 = center + (double)first * (double)spacing, c1 = c0 + (double)(n - 1) * (double)spacing;
+      const double reach = (c0 < (double)(ncol - 1) - c1 ? c0 : (double)(ncol - 1) - c1) - 1e-2;
+      // (nor where hardly a block lies within the reach)
+      if (!always && !(centers_worth(n, nrow, ncol) && reach > 0.125 * (double)ncol)) break;
+      if (first == 0) {
+        if (cudaMemsetAsync(workspace, 0, kHeader, st) != cudaSuccess)
+          return atb::fail(ATB_ECUDA, "atb_backproject_centers_stack: %s", cudaGetErrorString(cudaGetLastError()));
+        absmax_kernel<float><<<dim3(nrow < 256 ? nrow : 256, 1), 256, 0, st>>>(sino, sino_row_stride, 0, nrow, ncol,
+                                                                              maxbits);
+        rc = atb::check_launch("atb_backproject_centers_stack (scan)");
+        if (rc != ATB_OK) return rc;
+      }
       // samples of the first centre's frame: later centres read further on
       pack_centers_kernel<<<dim3((ncol + 255) / 256, nrow, S / 8), 256, 0, st>>>(sino, sino_row_stride, ncol, n, S,
                                                                                 spacing, first == 0, maxbits, packed);
@@ -991,7 +1039,6 @@ extern "C" int atb_backproject_centers_stack(const float *sino, int64_t sino_row
       a.nrow = nrow; a.ncol = ncol; a.nsl = n;
       a.center = c0; a.edge_pad = edge_pad ? 1 : 0; a.mask_r2 = mask_r2; a.scale = scale;
       a.out = out + (int64_t)first * out_center_stride; a.ors = out_row_stride; a.oss = out_center_stride;
-      const double reach = (c0 < (double)(ncol - 1) - c1 ? c0 : (double)(ncol - 1) - c1) - 1e-2;
       a.interior = reach > 0.0 ? reach : 0.0;
       a.inject = 0;
       rc = launch(a, S, packed, st);

@@ -215,8 +215,8 @@ int atb_backproject(const void *sino, int sino_dtype, int64_t sino_row_stride,
 
 /*
  * atb_backproject, given a workspace.  Stacks of 15 and more
- * float32 or float16 slices run on the tensor cores, up to 32 slices per
- * launch: samples and weights are split in two float16 terms each and the sums
+ * float32 or float16 slices run on the tensor cores where they are the faster
+ * (24 to 320 angles and more, by slices and size), up to 32 slices per launch: samples and weights are split in two float16 terms each and the sums
  * are compensated FP32.  A sample is held to 22 bits down to 2^-17 of its
  * slice's largest, so that results differ from atb_backproject's by rounding
  * only.  Where a slice holds more pairs of neighbouring samples below about
@@ -228,7 +228,9 @@ int atb_backproject(const void *sino, int sino_dtype, int64_t sino_row_stride,
  *
  *   flags      bit 4 as atb_backproject (the same results); bit 5 (tests only):
  *              the first CTA's first copies are armed for 16 bytes more than
- *              they deliver, and it gives up; else 0
+ *              they deliver, and it gives up; bit 6 (tests only): the tensor
+ *              cores also for groups with so few angles that atb_backproject
+ *              is the faster; else 0
  *   workspace  128-byte aligned device scratch of
  *              atb_backproject_stack_workspace bytes (0: none is used), free
  *              for reuse when the call's work on the stream is done
@@ -276,10 +278,10 @@ int atb_backproject_centers(const float *sino, int64_t sino_row_stride,
 /*
  * atb_backproject_centers, given a workspace: groups of 15 and more centres run
  * on the tensor cores (up to 32 per launch) where no position leaves the
- * detector for any of them, the rest of the image, sinograms of the kind that
- * atb_backproject_stack leaves to atb_backproject, and every call without a
- * (large enough) workspace as atb_backproject_centers does.  Results differ by
- * rounding only.
+ * detector for any of them, and where that is the faster; the rest of the image,
+ * sinograms of the kind that atb_backproject_stack leaves to atb_backproject, and
+ * every call without a (large enough) workspace as atb_backproject_centers does.
+ * Results differ by rounding only.  flags: bits 4 and 6 as atb_backproject_stack.
  *
  *   workspace  128-byte aligned device scratch of
  *              atb_backproject_centers_workspace bytes (0: none is used)

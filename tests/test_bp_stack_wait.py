@@ -4,7 +4,7 @@
 copies for 16 bytes more than they deliver: every copy completes, nothing is
 withheld, and the waits for them run out after their second.  The CTA then
 requests nothing more (a ring slot short of bytes must not be armed again) and
-walks to its end; the call returns, the status word says so, only that region of
+walks to its end (bit 6: whatever the angles); the call returns, the status word says so, only that region of
 16 x 16 pixels is missing, and the next call is right.
 """
 import numpy as np
@@ -35,7 +35,7 @@ def test_wait_runs_out_and_is_reported(cuda, nrow, nslice, edge_pad):
         nat.call("atb_backproject_stack", s3.data_ptr(), nat.F32,
                  s3.stride(0), s3.stride(1), nrow, nslice, ncol,
                  trig.data_ptr(), 39.25, edge_pad, -1.0, 1.0, out.data_ptr(),
-                 out.stride(0), out.stride(1), flags, ws.data_ptr(), need,
+                 out.stride(0), out.stride(1), flags | 64, ws.data_ptr(), need,
                  R._stream_ptr(cuda))
         torch.cuda.synchronize()
         return out
