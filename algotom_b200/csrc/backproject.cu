@@ -1029,8 +1029,9 @@ __global__ void __launch_bounds__(256) sum_groups_kernel(BPArgs a) {
 }
 
 // Angles per CTA when a launch's tiles do not fill the GPU evenly: nrow (no
-// groups), or a multiple of the chunk.  The rule is read off a sweep of 1 to 24
-// groups (us; masked disc, sum of the groups included), whose optima are broad:
+// groups), or a multiple of the chunk.  The most groups that can help are read off
+// a sweep of 1 to 24 groups (us; masked disc, sum of the groups included), whose
+// optima are broad:
 //   64 x 64, one slice   1200 x 1536: 1155 (1), 970 (6), 935 (8), 974 (24)
 //                        1801 x 2560: 3755 (1), 3355 (6), 3462 (16)
 //   32 x 32, one slice   181 x 256: 75 (1), 48 (6); 400 x 400: 144 (1), 86 (6),
@@ -1040,17 +1041,45 @@ __global__ void __launch_bounds__(256) sum_groups_kernel(BPArgs a) {
 //   two slices           900 x 512: 430 (1), 234 (10); x 1024: 856 (1), 681 (6)
 //   four slices          300 x 300: 218 (1), 88 (8); 900 x 800: 744 (1), 705 (6)
 //   eight (two CTA layers of four): 900 x 1024: 1996 (1), 2018 (4)
+// A group costs its partial image, whatever its angles, and earns a share of the
+// time that CTAs would stand idle in (mostly the last wave), so that few angles
+// bear few groups or none: at most a group for each angle times (0.1 idle share +
+// 0.005), 0.01 for the larger tiles, whose CTAs end unevenly.  Times without, with
+// the groups above alone, and with this rule (no mask):
+//   one slice    120 x 1024: 82, 91, 82; 361 x 1024: 243, 217, 217; 181 x 2560:
+//                440, 527, 440; 720 x 2560: 1688, 1655, 1655
+//   two          120 x 1024: 125, 181, 125; 361 x 1024: 350, 361, 339; 181 x 1536:
+//                342, 392, 342
+//   four, eight  181 x 800: 259, 210, 206; 65 x 1024: 113, 147, 113; 65 x 640 (8):
+//                111, 138, 111
+// Of 780 combinations none is over 1.07 of the better of the first two.
 template <typename T, int S, int V>
 int group_rows(int nrow, int nslices, int ncol) {
   using K = BPCfg<T, S, V>;
   const long long tiles =
       (long long)((ncol + K::TX - 1) / K::TX) * ((ncol + K::TY - 1) / K::TY) * ((nslices + S - 1) / S);
   const int nchunk = (nrow + K::kChunk - 1) / K::kChunk;
+  constexpr long long slots = 148 * K::kMinBlocks;
+  const double idle = 1.0 - (double)tiles / (double)((tiles + slots - 1) / slots * slots);
   long long g;
-  if (S == 1 && V == 1) g = tiles > 3000 ? 1 : std::min(16ll, std::max(5ll, 11000 / tiles));
-  else if (S == 1) g = tiles > 3000 ? 1 : std::min(12ll, std::max(6ll, 4500 / tiles));
-  else if (S == 2) g = tiles > 1500 ? 1 : std::min(10ll, std::max(4ll, 4500 / tiles));
-  else g = tiles > 600 ? 1 : std::min(8ll, 2000 / tiles);
+  double angles_per_tile, base = 0.005;
+  if (S == 1 && V == 1) {
+    g = tiles > 1700 ? 1 : std::min(16ll, std::max(5ll, 11000 / tiles));
+    angles_per_tile = 0.15;
+  } else if (S == 1) {
+    g = tiles > 3000 || nrow < 300 ? 1 : std::min(12ll, std::max(6ll, 4500 / tiles));
+    angles_per_tile = 0.3;
+    base = 0.01;
+  } else if (S == 2) {
+    g = tiles > 1500 ? 1 : std::min(10ll, std::max(4ll, 4500 / tiles));
+    angles_per_tile = 0.36;
+  } else {
+    g = tiles > 600 ? 1 : std::min(8ll, 2000 / tiles);
+    angles_per_tile = 0.36;
+  }
+  if ((double)nrow < angles_per_tile * (double)tiles) return nrow;
+  g = std::min(g, (long long)((double)nrow * (0.1 * idle + base)));
+  if (g < 3) return nrow;
   g = std::min(g, (long long)nchunk);
   return g <= 1 ? nrow : (int)((nchunk + g - 1) / g * K::kChunk);
 }
@@ -1105,7 +1134,10 @@ int launch_bp(BPArgs a, int nslices, cudaStream_t st, float2 *work = nullptr) {
 template <typename T>
 int dispatch(BPArgs a, int per_angle_kahan, int variant, cudaStream_t st, float2 *work) {
   if (per_angle_kahan) return launch_bp<T, 1, true>(a, a.nslice, st);
-  if (work) variant = split_variant(a.ncol);
+  if (work && (a.nslice & 1)) {  // the single slice's tiles where it is split
+    const int v = split_variant(a.ncol);
+    if ((v ? group_rows<T, 1, 1>(a.nrow, 1, a.ncol) : group_rows<T, 1, 0>(a.nrow, 1, a.ncol)) < a.nrow) variant = v;
+  }
   if (a.nslice == 1 && variant == 1) return launch_bp<T, 1, false, 1>(a, 1, st, work);
   // four slices per CTA for the bulk of a stack, then the remainder
   const int n4 = (a.nslice / 4) * 4;
