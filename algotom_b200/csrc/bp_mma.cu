@@ -795,23 +795,28 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
+// The packed samples as a tensor: false where the driver has no tensor maps, and
+// the gather kernel takes the stack (as it stages without them).
+bool packed_map(int S, int nrow, int ncol, void *packed, CUtensorMap *map) {
+  auto encode = tensor_map_encoder();
+  std::memset(map, 0, sizeof(*map));
+  const cuuint64_t G = (cuuint64_t)S / 4;
+  const cuuint64_t dims[3] = {(cuuint64_t)ncol * 8, G, (cuuint64_t)nrow};
+  const cuuint64_t strides[2] = {(cuuint64_t)ncol * 16, (cuuint64_t)ncol * 16 * G};
+  const cuuint32_t box[3] = {kBins * 8, (cuuint32_t)G, 1u};
+  const cuuint32_t estr[3] = {1u, 1u, 1u};
+  return encode && encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, packed, dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <int S, int F>
-int launch_mma(const MmaArgs &a, void *packed, cudaStream_t st) {
+int launch_mma(const MmaArgs &a, const CUtensorMap &map, cudaStream_t st) {
   using K = MmaCfg<S>;
+  static_assert(K::G == S / 4, "as packed_map");
   auto fn = bp_mma_kernel<S, F>;
   const int rc = atb::ensure_smem(fn, K::kSmem, "atb_backproject_stack", kThreads, 512);
   if (rc != ATB_OK) return rc;
-  auto encode = tensor_map_encoder();
-  CUtensorMap map;
-  std::memset(&map, 0, sizeof(map));
-  const cuuint64_t dims[3] = {(cuuint64_t)a.ncol * 8, (cuuint64_t)K::G, (cuuint64_t)a.nrow};
-  const cuuint64_t strides[2] = {(cuuint64_t)a.ncol * 16, (cuuint64_t)a.ncol * 16 * K::G};
-  const cuuint32_t box[3] = {kBins * 8, (cuuint32_t)K::G, 1u};
-  const cuuint32_t estr[3] = {1u, 1u, 1u};
-  if (!encode || encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, packed, dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return atb::fail(ATB_ECUDA, "atb_backproject_stack: no tensor map");
   const int n = (a.ncol + kRegion - 1) / kRegion;
   fn<<<dim3(n, n), kThreads, K::kSmem, st>>>(a, map);
   return atb::check_launch("atb_backproject_stack");
@@ -834,14 +839,14 @@ int fold_steps(const MmaArgs &a) {
   return a.edge_pad || (long long)a.ncol * a.ncol < 600ll * a.nrow ? kFoldShort : kFoldLong;
 }
 
-int launch(const MmaArgs &a, int S, void *packed, cudaStream_t st) {
+int launch(const MmaArgs &a, int S, const CUtensorMap &map, cudaStream_t st) {
   if (fold_steps(a) == kFoldShort)
-    return S == 16   ? launch_mma<16, kFoldShort>(a, packed, st)
-           : S == 24 ? launch_mma<24, kFoldShort>(a, packed, st)
-                     : launch_mma<32, kFoldShort>(a, packed, st);
-  return S == 16   ? launch_mma<16, kFoldLong>(a, packed, st)
-         : S == 24 ? launch_mma<24, kFoldLong>(a, packed, st)
-                   : launch_mma<32, kFoldLong>(a, packed, st);
+    return S == 16   ? launch_mma<16, kFoldShort>(a, map, st)
+           : S == 24 ? launch_mma<24, kFoldShort>(a, map, st)
+                     : launch_mma<32, kFoldShort>(a, map, st);
+  return S == 16   ? launch_mma<16, kFoldLong>(a, map, st)
+         : S == 24 ? launch_mma<24, kFoldLong>(a, map, st)
+                   : launch_mma<32, kFoldLong>(a, map, st);
 }
 
 template <typename T>
@@ -943,9 +948,9 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
                                      double center, int edge_pad, double mask_r2, float scale, float *out,
                                      int64_t out_row_stride, int64_t out_slice_stride, int flags, void *workspace,
                                      int64_t workspace_bytes, void *stream) {
-  if (flags & ~112) return atb::fail(ATB_EINVAL, "atb_backproject_stack: unknown flags %d", flags);
-  const bool always = flags & 64;
-  flags &= ~64;
+  if (flags & ~240) return atb::fail(ATB_EINVAL, "atb_backproject_stack: unknown flags %d", flags);
+  const bool always = flags & 64, no_maps = flags & 128;
+  flags &= ~192;
   cudaStream_t st = atb::as_stream(stream);
   const int64_t need = atb_backproject_stack_workspace(sino_dtype, nrow, nslice, ncol);
   const int esize = sino_dtype == ATB_F32 ? 4 : 2;
@@ -957,6 +962,9 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
     for (int n; (n = next_group(sino_dtype, nrow, ncol, nslice - first)) > 0; first += n) {
       if (!always && nrow < fewest_angles(n, ncol)) break;
       const int S = padded(n);
+      void *packed = static_cast<unsigned char *>(workspace) + kHeader;
+      CUtensorMap map;
+      if (no_maps || !packed_map(S, nrow, ncol, packed, &map)) break;
       const char *src = static_cast<const char *>(sino) + (int64_t)first * sino_slice_stride * esize;
       float *dst = out + (int64_t)first * out_slice_stride;
       int rc = sino_dtype == ATB_F32
@@ -972,7 +980,7 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
       a.out = dst; a.ors = out_row_stride; a.oss = out_slice_stride;
       a.interior = -1.0;
       a.inject = (flags >> 5) & 1;
-      rc = launch(a, S, static_cast<unsigned char *>(workspace) + kHeader, st);
+      rc = launch(a, S, map, st);
       if (rc != ATB_OK) return rc;
       // runs only where bp_left_to_gather
       rc = atb::bp_gather(src, sino_dtype, sino_row_stride, sino_slice_stride, nrow, n, ncol, trig, center, edge_pad,
@@ -1018,6 +1026,8 @@ extern "C" int atb_backproject_centers_stack(const float *sino, int64_t sino_row
       const double reach = (c0 < (double)(ncol - 1) - c1 ? c0 : (double)(ncol - 1) - c1) - 1e-2;
       // (nor where hardly a block lies within the reach)
       if (!always && !(centers_worth(n, nrow, ncol) && reach > 0.125 * (double)ncol)) break;
+      CUtensorMap map;
+      if (!packed_map(S, nrow, ncol, packed, &map)) break;
       if (first == 0) {
         if (cudaMemsetAsync(workspace, 0, kHeader, st) != cudaSuccess)
           return atb::fail(ATB_ECUDA, "atb_backproject_centers_stack: %s", cudaGetErrorString(cudaGetLastError()));
@@ -1041,7 +1051,7 @@ extern "C" int atb_backproject_centers_stack(const float *sino, int64_t sino_row
       a.out = out + (int64_t)first * out_center_stride; a.ors = out_row_stride; a.oss = out_center_stride;
       a.interior = reach > 0.0 ? reach : 0.0;
       a.inject = 0;
-      rc = launch(a, S, packed, st);
+      rc = launch(a, S, map, st);
       if (rc != ATB_OK) return rc;
       // the blocks whose positions reach an edge of the detector for some
       // centre: each centre has its own edges there

@@ -230,7 +230,8 @@ int atb_backproject(const void *sino, int sino_dtype, int64_t sino_row_stride,
  *              the first CTA's first copies are armed for 16 bytes more than
  *              they deliver, and it gives up; bit 6 (tests only): the tensor
  *              cores also for groups with so few angles that atb_backproject
- *              is the faster; else 0
+ *              is the faster; bit 7 (tests only): as where the driver encodes
+ *              no tensor maps; else 0
  *   workspace  128-byte aligned device scratch of
  *              atb_backproject_stack_workspace bytes (0: none is used), free
  *              for reuse when the call's work on the stream is done

@@ -108,6 +108,15 @@ def test_groups_with_few_angles_take_the_gather_kernel(cuda, nrow, nslice,
         assert torch.equal(got[:, tensor:], gather)
 
 
+def test_without_tensor_maps_the_gather_kernel_runs(cuda):
+    """(bit 7: the driver's encoder is not there)"""
+    nrow, nslice, ncol = 90, 33, 100
+    ang = np.linspace(0.0, np.pi, nrow)
+    t = torch.from_numpy(_stack(nrow, nslice, ncol)).to(cuda)
+    got = _bp("atb_backproject_stack", t, ang, 48.75, True, 128)
+    assert torch.equal(got, _bp("atb_backproject", t, ang, 48.75, True))
+
+
 @pytest.mark.parametrize("nrow,ncol,n,c0,tensor", [
     (400, 96, 16, 40.5, 0), (23, 96, 15, 40.5, 0), (24, 96, 15, 40.5, 15),
     (127, 400, 20, 190.5, 0), (128, 400, 20, 190.5, 20),
