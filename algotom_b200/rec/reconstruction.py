@@ -158,20 +158,21 @@ def filter_sinograms(sino3, pad, pad_mode="edge", apply_log=False,
 
 
 def backproject(sino3, angles, center, edge_pad=False, mask_r2=-1.0,
-                scale=1.0, out=None, kahan="chunk", trig=None, variant=0,
+                scale=1.0, out=None, kahan="chunk", trig=None, variant=None,
                 staging="tma"):
     """Device back-projection of [nrow, nslice, ncol] -> [ncol, nslice, ncol].
 
     ``sino3`` may be float32, float16 or bfloat16 (last axis contiguous).
     ``trig`` may hold the angle table from :func:`_trig` already on the
-    device (saves its host-to-device copy per call).  ``variant`` selects
-    the single-slice tile variant (0: 64 x 64, 1: 32 x 32).  ``staging``:
+    device (saves its host-to-device copy per call).  ``variant`` 0
+    or 1 asks for ``atb_backproject`` with that single-slice tile variant (0:
+    64 x 64, 1: 32 x 32), without angle groups or tensor cores.  ``staging``:
     "tma" stages the detector windows of 2- and 4-slice CTAs with TMA box
     loads where the rows are 16-byte aligned, "cp.async" always with
-    cp.async; the results are the same.  Unless ``kahan`` is "angle", stacks
-    of 15 and more slices (not bfloat16) run on the tensor cores, and launches
-    with few tiles split the angles over more CTAs, ``variant`` or not
-    (``atb_backproject_stack``).
+    cp.async; the results are the same.  By default, unless ``kahan`` is
+    "angle", stacks of 15 and more slices (not bfloat16) run on the tensor cores
+    where that is the faster, and launches with few tiles split the angles over
+    more CTAs (``atb_backproject_stack``).
     """
     if staging not in ("tma", "cp.async"):
         raise ValueError("staging must be 'tma' or 'cp.async'")
@@ -183,7 +184,7 @@ def backproject(sino3, angles, center, edge_pad=False, mask_r2=-1.0,
     if out is None:
         out = torch.empty((ncol, nslice, ncol), dtype=torch.float32,
                           device=dev)
-    if kahan != "angle":
+    if kahan != "angle" and variant is None:
         need = _stack_need(code, nrow, nslice, ncol)
         if need > 0:
             ws = _stack_workspace(need, dev)
@@ -200,7 +201,7 @@ def backproject(sino3, angles, center, edge_pad=False, mask_r2=-1.0,
              sino3.stride(1), nrow, nslice, ncol, trig.data_ptr(),
              float(np.float32(center)), int(bool(edge_pad)), float(mask_r2),
              float(scale), out.data_ptr(), out.stride(0), out.stride(1),
-             (1 if kahan == "angle" else 0) | (int(variant) << 2) |
+             (1 if kahan == "angle" else 0) | (int(variant or 0) << 2) |
              (16 if staging == "cp.async" else 0), _stream_ptr(dev))
     return out
 
