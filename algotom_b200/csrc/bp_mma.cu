@@ -935,11 +935,14 @@ extern "C" int64_t atb_backproject_stack_workspace(int sino_dtype, int nrow, int
   if (nrow < 1 || nslice < 1 || ncol < 1 || nrow > 65535 || ncol > (1 << 16)) return 0;
   const int n = next_group(sino_dtype, nrow, ncol, nslice);
   const int64_t packed = n ? kHeader + (int64_t)nrow * ncol * padded(n) * 4 : 0;
-  // slices left over after the last launch of the tensor cores
-  int left = nslice;
-  if (n == 32) left %= 32;
-  if (next_group(sino_dtype, nrow, ncol, left)) left = 0;
-  const int64_t split = left ? atb::bp_gather_workspace(nrow, left, ncol) : 0;
+  // the gather kernel's angle groups: of 32 slices, and of what is left over
+  const int left = nslice % 32;
+  int64_t split = 0;
+  if (left && !next_group(sino_dtype, nrow, ncol, left)) split = atb::bp_gather_workspace(nrow, left, ncol);
+  if (nslice >= 32 && n == 0) {
+    const int64_t whole = atb::bp_gather_workspace(nrow, 32, ncol);
+    if (whole > split) split = whole;
+  }
   return packed > split ? packed : split;
 }
 
@@ -988,13 +991,30 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
       if (rc != ATB_OK) return rc;
     }
     if (first == nslice) return ATB_OK;
+    // the gather kernel: whole launches of 32 slices, then the rest, so that a
+    // slice's bits depend on its place among them and not on how many follow
+    auto gather = [&](int n, bool split) {
+      const int rc = atb::bp_gather(static_cast<const char *>(sino) + (int64_t)first * sino_slice_stride * esize,
+                                    sino_dtype, sino_row_stride, sino_slice_stride, nrow, n, ncol, trig, center,
+                                    edge_pad, mask_r2, scale, out + (int64_t)first * out_slice_stride, out_row_stride,
+                                    out_slice_stride, flags, nullptr, split ? workspace : nullptr, stream);
+      first += n;
+      return rc;
+    };
+    int whole = (nslice - first) / 32 * 32;
+    // (without angle groups one launch gives the same bits)
+    const bool split = next_group(sino_dtype, nrow, ncol, 32) == 0 && atb::bp_gather_workspace(nrow, 32, ncol) > 0;
+    while (whole > 0) {
+      const int n = split ? 32 : whole;
+      const int rc = gather(n, split);
+      if (rc != ATB_OK) return rc;
+      whole -= n;
+    }
+    const int left = nslice - first;
+    return left ? gather(left, next_group(sino_dtype, nrow, ncol, left) == 0) : ATB_OK;
   }
-  // (the workspace is sized for the angle groups of what next_group leaves)
-  if (work_ok && next_group(sino_dtype, nrow, ncol, nslice - first)) workspace = nullptr;
-  return atb::bp_gather(args_ok ? static_cast<const char *>(sino) + (int64_t)first * sino_slice_stride * esize : sino,
-                        sino_dtype, sino_row_stride, sino_slice_stride, nrow, nslice - first, ncol, trig, center,
-                        edge_pad, mask_r2, scale, out ? out + (int64_t)first * out_slice_stride : out, out_row_stride,
-                        out_slice_stride, flags, nullptr, work_ok ? workspace : nullptr, stream);
+  return atb::bp_gather(sino, sino_dtype, sino_row_stride, sino_slice_stride, nrow, nslice, ncol, trig, center, edge_pad,
+                        mask_r2, scale, out, out_row_stride, out_slice_stride, flags, nullptr, nullptr, stream);
 }
 
 extern "C" int64_t atb_backproject_centers_workspace(int nrow, int ncol, int ncenter) {

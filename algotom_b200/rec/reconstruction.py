@@ -377,20 +377,41 @@ def _slab_spans(nslice, slab):
     """(first slice, count) of the slabs of a streamed stack: full slabs of
     ``slab``, with the first and last ramped (slab/4, slab/4, slab/2) so the
     copy-in that nothing overlaps before the first kernel and the copy-out
-    after the last one are short."""
+    after the last one are short; what is left over comes last, so that no
+    slab crosses a multiple of ``slab``."""
     ramp = [max(1, slab // 4), max(1, slab // 4), max(1, slab // 2)]
-    if nslice < 2 * slab + 2 * sum(ramp):
-        sizes = [slab] * (nslice // slab) + ([nslice % slab]
-                                            if nslice % slab else [])
+    left = [nslice % slab] if nslice % slab else []
+    if nslice < 2 * slab + 2 * sum(ramp) or sum(ramp) != slab:
+        sizes = [slab] * (nslice // slab) + left
     else:
-        mid = nslice - 2 * sum(ramp)
-        sizes = ramp + [slab] * (mid // slab) + \
-            ([mid % slab] if mid % slab else []) + ramp[::-1]
+        sizes = ramp + [slab] * (nslice // slab - 2) + ramp[::-1] + left
     spans, k0 = [], 0
     for n in sizes:
         spans.append((k0, n))
         k0 += n
     return spans
+
+
+def _slab_groups(spans, slab, nrow, ncol, storage, kahan):
+    """The slabs that go through the kernels together, as lists of spans.
+
+    Where :func:`backproject` takes whole slabs another way than their parts
+    (the tensor cores, which cost about the same for 16 as for 32 slices; angle
+    groups), the ramps' slabs are joined: the streamed results then have the
+    bits of the device-resident ones, whose launches end at the same slices.
+    Elsewhere every span goes by itself."""
+    code = _STORAGE[storage][1]
+    left = sum(n for _, n in spans) % slab  # the last span, which joins none
+    sizes = {slab} | {n for _, n in (spans[:-1] if left else spans)}
+    join = kahan != "angle" and any(_stack_need(code, nrow, n, ncol) > 0
+                                    for n in sizes)
+    groups = []
+    for sp in spans:
+        if join and groups and sum(n for _, n in groups[-1]) + sp[1] <= slab:
+            groups[-1].append(sp)
+        else:
+            groups.append([sp])
+    return groups
 
 
 def _resume_key(shape, center, angles, mask_r2, scale, ramp_win,
@@ -417,17 +438,20 @@ def _fbp_streamed(host, center, angles, mask_r2, scale, ramp_win, filter_name,
                   pad, pad_mode, apply_log, out_host, storage, kahan,
                   slab=SLAB, manifest=None):
     """FBP of a host stack [nrow, nslice, ncol] streamed through the device
-    in slabs of up to ``slab`` slices (ramped at both ends): while slab k is
-    filtered and back-projected, slab k+1 is copied in and slab k-1 copied
-    out (one copy stream each way, double-buffered, ordered by events).
-    With a :class:`~algotom_b200.rec.resume.SlabManifest`, slabs it lists
-    are skipped and every slab whose copy-out has completed is recorded."""
+    in slabs of up to ``slab`` slices (:func:`_slab_spans`,
+    :func:`_slab_groups`): while slab k is filtered and back-projected, slab
+    k+1 is copied in and slab k-1 copied out (one copy stream each way,
+    double-buffered, ordered by events).  With a
+    :class:`~algotom_b200.rec.resume.SlabManifest`, slabs it lists are skipped
+    and every slab whose copy-out has completed is recorded."""
     nrow, nslice, ncol = host.shape
     dev = _device()
     k_sl = max(1, min(slab, nslice))
-    spans = _slab_spans(nslice, k_sl)
+    groups = _slab_groups(_slab_spans(nslice, k_sl), k_sl, nrow, ncol,
+                          storage, kahan)
     if manifest is not None:
-        spans = [sp for sp in spans if not manifest.is_done(sp)]
+        groups = [g for g in groups
+                  if not all(manifest.is_done(sp) for sp in g)]
     pending = []  # (copy-out event, span) not yet recorded as finished
     cmp = torch.cuda.current_stream(dev)
     s_in, s_out = torch.cuda.Stream(dev), torch.cuda.Stream(dev)
@@ -447,7 +471,8 @@ def _fbp_streamed(host, center, angles, mask_r2, scale, ramp_win, filter_name,
     hp, op = host.data_ptr(), out_host.data_ptr()
     trig = _trig(angles, dev)
     cmp.synchronize()
-    for k, (k0, kk) in enumerate(spans):
+    for k, group in enumerate(groups):
+        k0, kk = group[0][0], sum(n for _, n in group)
         b = k % 2
         if manifest is not None and pending:
             fin = [sp for ev, sp in pending if ev.query()]
@@ -475,7 +500,7 @@ def _fbp_streamed(host, center, angles, mask_r2, scale, ramp_win, filter_name,
         if manifest is not None:
             done = torch.cuda.Event()
             done.record(s_out)
-            pending.append((done, (k0, kk)))
+            pending.extend((done, sp) for sp in group)
         del f
     s_out.synchronize()
     s_in.synchronize()

@@ -110,7 +110,7 @@ def test_groups_with_few_angles_take_the_gather_kernel(cuda, nrow, nslice,
 
 def test_without_tensor_maps_the_gather_kernel_runs(cuda):
     """(bit 7: the driver's encoder is not there)"""
-    nrow, nslice, ncol = 90, 33, 100
+    nrow, nslice, ncol = 90, 32, 100
     ang = np.linspace(0.0, np.pi, nrow)
     t = torch.from_numpy(_stack(nrow, nslice, ncol)).to(cuda)
     got = _bp("atb_backproject_stack", t, ang, 48.75, True, 128)
