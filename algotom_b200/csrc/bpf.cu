@@ -141,11 +141,17 @@ __device__ double pad_value(const BpfArgs &a, const float *X, int ks, int ry, in
 // as fill the register file.
 constexpr int fft_threads(bool big) { return big ? 512 : 768; }
 
+// LEAN: with those passes.  Riding on the stages makes three copies of every
+// radix's code, and a launch of few CTAs is over before it has fetched it: one
+// slice of 100 pixels 22 us with the passes, 33 without; four of 200, 38 and 43; one
+// of 300, 38 and 45; four of 300, 55 and 53; sixteen of 100, 49 and 42.
+constexpr long long kLeanCtas = 600;
+
 // Grids put the slice pair on x, so that the CTAs of one row / column of
 // every pair run together (the columns kernel then reads each spectrum
 // column once from DRAM).  Shared memory: two buffers of T values, then
 // the twiddle table.
-template <bool BIG>
+template <bool BIG, bool LEAN>
 __global__ void __launch_bounds__(fft_threads(BIG), 1) bpf_rows_kernel(BpfArgs a, const __grid_constant__ Plan pl) {
   extern __shared__ double2 sm[];
   const int ry = blockIdx.y, g = blockIdx.x, T = pl.n;
@@ -165,51 +171,75 @@ __global__ void __launch_bounds__(fft_threads(BIG), 1) bpf_rows_kernel(BpfArgs a
   }
   __syncthreads();
   double2 *w = a.work + ((long long)g * a.n + ry) * T;
-  atb::fft::run_io<false, BIG>(sm, sm + T, pl, tws, atb::fft::FromBuffer(),
-                               [w](double2 *, int kx, double2 v) { w[kx] = v; });
+  if constexpr (LEAN) {
+    const double2 *res = atb::fft::run<false, BIG>(sm, sm + T, pl, tws);
+    for (int kx = threadIdx.x; kx < T; kx += blockDim.x) w[kx] = res[kx];
+  } else {
+    atb::fft::run_io<false, BIG>(sm, sm + T, pl, tws, atb::fft::FromBuffer(),
+                                 [w](double2 *, int kx, double2 v) { w[kx] = v; });
+  }
 }
 
-template <bool BIG>
+template <bool BIG, bool LEAN>
 __global__ void __launch_bounds__(fft_threads(BIG), 1) bpf_cols_kernel(BpfArgs a, const __grid_constant__ Plan pl) {
   extern __shared__ double2 sm[];
   const int kx = blockIdx.y, g = blockIdx.x, T = pl.n, n = a.n;
   double2 *tws = sm + 2 * T;
   atb::fft::load_twiddles(pl, tws);
   double2 *w = a.work + (long long)g * n * T + kx;
-  __syncthreads();
   const bool cplx = a.spec_complex;
   const double2 *Sc = static_cast<const double2 *>(a.spec) + (long long)kx * T;
   const double *Sr = static_cast<const double *>(a.spec) + (long long)kx * T;
-  double2 *res = atb::fft::run_io<false, BIG>(
-      sm, sm + T, pl, tws,
-      [w, n, T](const double2 *, int ry) { return ry < n ? w[(long long)ry * T] : make_double2(0.0, 0.0); },
-      [cplx, Sc, Sr](double2 *buf, int ky, double2 v) {
-        if (cplx) {
-          v = atb::fft::cmul(v, __ldg(Sc + ky));
-        } else {
-          const double h = __ldg(Sr + ky);
-          v.x *= h;
-          v.y *= h;
-        }
-        buf[ky] = v;
-      });
   const int u0 = a.pad, u1 = a.pad + a.ncol;
-  atb::fft::run_io<true, BIG>(res, res == sm ? sm + T : sm, pl, tws, atb::fft::FromBuffer(),
-                              [w, T, u0, u1](double2 *, int u, double2 v) {
-                                if (u >= u0 && u < u1) w[(long long)u * T] = v;
-                              });
+  const auto load = [w, n, T](const double2 *, int ry) {
+    return ry < n ? w[(long long)ry * T] : make_double2(0.0, 0.0);
+  };
+  const auto times = [cplx, Sc, Sr](double2 *buf, int ky, double2 v) {
+    if (cplx) {
+      v = atb::fft::cmul(v, __ldg(Sc + ky));
+    } else {
+      const double h = __ldg(Sr + ky);
+      v.x *= h;
+      v.y *= h;
+    }
+    buf[ky] = v;
+  };
+  const auto store = [w, T, u0, u1](double2 *, int u, double2 v) {
+    if (u >= u0 && u < u1) w[(long long)u * T] = v;
+  };
+  if constexpr (LEAN) {
+    for (int ry = threadIdx.x; ry < T; ry += blockDim.x) sm[ry] = load(sm, ry);
+    __syncthreads();
+    double2 *res = atb::fft::run<false, BIG>(sm, sm + T, pl, tws);
+    double2 *other = res == sm ? sm + T : sm;
+    for (int ky = threadIdx.x; ky < T; ky += blockDim.x) times(res, ky, res[ky]);
+    __syncthreads();
+    const double2 *out = atb::fft::run<true, BIG>(res, other, pl, tws);
+    for (int u = u0 + threadIdx.x; u < u1; u += blockDim.x) w[(long long)u * T] = out[u];
+  } else {
+    __syncthreads();
+    double2 *res = atb::fft::run_io<false, BIG>(sm, sm + T, pl, tws, load, times);
+    atb::fft::run_io<true, BIG>(res, res == sm ? sm + T : sm, pl, tws, atb::fft::FromBuffer(), store);
+  }
 }
 
-template <bool BIG>
+template <bool BIG, bool LEAN>
 __global__ void __launch_bounds__(fft_threads(BIG), 1) bpf_out_kernel(BpfArgs a, const __grid_constant__ Plan pl) {
   extern __shared__ double2 sm[];
   const int y = blockIdx.y, g = blockIdx.x, T = pl.n;
   double2 *tws = sm + 2 * T;
   atb::fft::load_twiddles(pl, tws);
   const double2 *w = a.work + ((long long)g * a.n + y + a.pad) * T;
-  __syncthreads();
-  const double2 *res = atb::fft::run_io<true, BIG>(
-      sm, sm + T, pl, tws, [w](const double2 *, int kx) { return w[kx]; }, atb::fft::ToBuffer());
+  const double2 *res;
+  if constexpr (LEAN) {
+    for (int kx = threadIdx.x; kx < T; kx += blockDim.x) sm[kx] = w[kx];
+    __syncthreads();
+    res = atb::fft::run<true, BIG>(sm, sm + T, pl, tws);
+  } else {
+    __syncthreads();
+    res = atb::fft::run_io<true, BIG>(
+        sm, sm + T, pl, tws, [w](const double2 *, int kx) { return w[kx]; }, atb::fft::ToBuffer());
+  }
   const int sa = a.slice0 + 2 * g, sb = sa + 1;
   const bool hb = sb < a.nslice;
   const int c = a.ncol / 2;
@@ -612,13 +642,17 @@ extern "C" int atb_bpf_filter2d(const float *src, int64_t src_row_stride, int64_
   bool big = false;
   for (int k = 0; k < pl.nstages; ++k) big = big || pl.radix[k] > 8;
   // the CTAs of an SM share its threads: of 128 where the shared memory holds five
-  // and more (four, BIG), else three (two), two or one
+  // and more (four, BIG) and the launch has them, else three (two), two or one
   const int fit = (int)std::max<size_t>(1, 228 * 1024 / (smem + 1024));
-  const int ctas = big ? (fit >= 4 ? 4 : std::min(2, fit)) : (fit >= 5 ? 6 : std::min(3, fit));
+  const bool lean = (long long)std::min(pairs, npairs) * (ncol + 2 * pad) < kLeanCtas;
+  const int ctas = big ? (fit >= 4 && !lean ? 4 : std::min(2, fit)) : (fit >= 5 && !lean ? 6 : std::min(3, fit));
   const int threads = fft_threads(big) / ctas;
-  const auto rows = big ? bpf_rows_kernel<true> : bpf_rows_kernel<false>;
-  const auto cols = big ? bpf_cols_kernel<true> : bpf_cols_kernel<false>;
-  const auto outs = big ? bpf_out_kernel<true> : bpf_out_kernel<false>;
+  const auto rows = lean ? (big ? bpf_rows_kernel<true, true> : bpf_rows_kernel<false, true>)
+                         : (big ? bpf_rows_kernel<true, false> : bpf_rows_kernel<false, false>);
+  const auto cols = lean ? (big ? bpf_cols_kernel<true, true> : bpf_cols_kernel<false, true>)
+                         : (big ? bpf_cols_kernel<true, false> : bpf_cols_kernel<false, false>);
+  const auto outs = lean ? (big ? bpf_out_kernel<true, true> : bpf_out_kernel<false, true>)
+                         : (big ? bpf_out_kernel<true, false> : bpf_out_kernel<false, false>);
   int rc = atb::ensure_smem(rows, smem, "atb_bpf_filter2d");
   if (rc == ATB_OK) rc = atb::ensure_smem(cols, smem, "atb_bpf_filter2d");
   if (rc == ATB_OK) rc = atb::ensure_smem(outs, smem, "atb_bpf_filter2d");

@@ -243,11 +243,11 @@ __device__ double2 *run_io(double2 *a, double2 *b, const Plan &pl, const double2
 // Transform of the n values in a[] (b[] is scratch of the same size; tws
 // the table of load_twiddles); returns the buffer holding the result.
 // Every thread of the CTA calls it.
-template <bool INV>
+template <bool INV, bool BIG = true>
 __device__ double2 *run(double2 *a, double2 *b, const Plan &pl, const double2 *tws) {
   int L = 1;
   for (int s = 0; s < pl.nstages; ++s) {
-    stage_of<INV, true>(pl.radix[s], a, b, pl, tws, L, FromBuffer(), ToBuffer());
+    stage_of<INV, BIG>(pl.radix[s], a, b, pl, tws, L, FromBuffer(), ToBuffer());
     __syncthreads();
     double2 *t = a;
     a = b;
