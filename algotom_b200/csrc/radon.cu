@@ -87,11 +87,7 @@ __device__ __forceinline__ double walk_bin(const float *src, long long rs, int v
   const float rf = (float)r;
   const double ic = 0.5 * (double)(ncol - 1);
   double acc = 0.0;
-  // weights of the three pixels from e = floor(u - span) - (u - span) in
-  // (-1, 0] and c = |cos| = 1 / span: their distances from the ray, in bins, are
-  // 1 - c - e c, |2 c - 1 + e c| and 3 c - 1 + e c (the first and the last keep
-  // their signs), so c + e c, 1 - |2 c - 1 + e c| and max(0, 2 - 3 c - e c)
-  const float c = fabsf(cf), c21 = fmaf(2.0f, c, -1.0f), c23 = fmaf(-3.0f, c, 2.0f);
+  const float c2 = 2.0f * cf, c3 = 3.0f * cf;
   for (int va = v0; va < v1; va += kRun) {
     const double X0 = fma((double)va, r, A);
     const double xid = floor(X0);
@@ -102,25 +98,28 @@ __device__ __forceinline__ double walk_bin(const float *src, long long rs, int v
     float run = 0.0f;
     if constexpr (!kEdge) {
       // a full run whose candidate pixels all lie inside the line: no bounds
-      // logic, and only the last weight can need its clamp at zero.  The first
-      // and the last step's t, formed as the loop forms them (t is monotonic in
-      // j), bound every index: rounded another way they may miss by a pixel.
-      const float xs = xf - spanf, te = fmaf((float)(kRun - 1), rf, xs);
-      if (nrun == kRun && xi + floor_small(fminf(xs, te)) + 1 >= 0 &&
-          xi + floor_small(fmaxf(xs, te)) + 3 <= ncol - 1) {
-        const float *base = line + xi - 0x4B400000ll + 1;
-        float run2 = 0.0f, run3 = 0.0f;
+      // logic, weights clamped at zero (a zero weight adds exactly 0, the same
+      // sum as the checked loop below).  The first and the last step's index,
+      // formed as the loop forms them (monotonic in j), bound the others; any
+      // other rounding could miss by a pixel.
+      const float xe = fmaf((float)(kRun - 1), rf, xf);
+      if (nrun == kRun && xi + floor_small(fminf(xf, xe) - spanf) + 1 >= 0 &&
+          xi + floor_small(fmaxf(xf, xe) - spanf) + 3 <= ncol - 1) {
+        const float *base = line + xi - 0x4B400000ll;
 #pragma unroll 8
         for (int j = 0; j < kRun; ++j, base += rs) {
-          const float t = fmaf((float)j, rf, xs);
-          const float tq = __fadd_rd(t, 12582912.0f);  // 0x4B400000 + floor(t) as an integer
-          const float e = (tq - 12582912.0f) - t;
+          const float xr = fmaf((float)j, rf, xf);
+          const float tq = __fadd_rd(xr - spanf, 12582912.0f);  // 0x4B400000 + floor(xr - span) as an integer
+          const float d0 = (tq - 12582912.0f) - xr;             // floor(xr - span) - xr
           const float *px = base + __float_as_int(tq);
-          run = fmaf(fmaf(e, c, c), __ldg(px), run);
-          run2 = fmaf(1.0f - fabsf(fmaf(e, c, c21)), __ldg(px + 1), run2);
-          run3 = fmaf(fmaxf(0.0f, fmaf(-e, c, c23)), __ldg(px + 2), run3);
+          const float w1 = __saturatef(1.0f - fabsf(fmaf(d0, cf, cf)));
+          const float w2 = __saturatef(1.0f - fabsf(fmaf(d0, cf, c2)));
+          const float w3 = __saturatef(1.0f - fabsf(fmaf(d0, cf, c3)));
+          run = fmaf(w1, __ldg(px + 1), run);
+          run = fmaf(w2, __ldg(px + 2), run);
+          run = fmaf(w3, __ldg(px + 3), run);
         }
-        acc += (double)(run + (run2 + run3));
+        acc += (double)run;
         continue;
       }
     }

@@ -2,8 +2,9 @@
 
 Rays whose run of 32 lines ends exactly on the first or last pixel: the end of
 the run, rounded as ``(xf + 31 r) - span``, is one pixel further in than as
-``(xf - span) + 31 r``, which is how the kernel walks.  The pixel beside the
-line carries next to no weight, so NaN around the image shows a read of it.
+``(xf - span) + 31 r``, so that bounds formed the one way do not hold a walk
+formed the other.  The pixel beside the line carries next to no weight, so NaN
+around the image shows a read of it.
 """
 import numpy as np
 import pytest
