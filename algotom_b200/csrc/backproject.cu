@@ -347,7 +347,7 @@ __host__ __device__ constexpr int group_segment(int win, int s, int spacing, int
   return ((win + (s - 1) * spacing + 3 * vec - 1) / vec) * vec;
 }
 
-template <typename T, int S, bool kPerAngleKahan, int V = 0, bool kGroup = false>
+template <typename T, int S, bool kPerAngleKahan, int V = 0, bool kGroup = false, bool kSplit = false>
 __device__ __forceinline__ void bp_tile(const BPArgs &a, int bx, int by, int bz, unsigned char *smem,
                                         uint32_t tmem, const CUtensorMap *tmap) {
   using K = BPCfg<T, S, V>;
@@ -383,7 +383,7 @@ __device__ __forceinline__ void bp_tile(const BPArgs &a, int bx, int by, int bz,
     const int cm = ncol / 2;
     const long long dx = max(0, max(x0 - cm, cm - (x0 + TX - 1))), dy = max(0, max(y0 - cm, cm - (y0 + TY - 1)));
     if ((double)(dx * dx + dy * dy) > a.mask_r2) {
-      if (!a.part) {
+      if constexpr (!kSplit) {
         for (int e = tid; e < TX * TY; e += kThreads) {
           const int x = x0 + e % TX, y = y0 + e / TX;
           if (x < ncol && y < ncol)
@@ -518,7 +518,8 @@ __device__ __forceinline__ void bp_tile(const BPArgs &a, int bx, int by, int bz,
         unsigned bytes = (unsigned)(kGroup ? seglen * (int)sizeof(T) : K::kBoxBytes);
         if (a.inject && k == 0 && tid == 0 && bx == 0 && by == 0 && bz == 0) bytes += 16u;
         mbar_arrive_expect_tx(&raw_bar, bytes);
-        tma_load_3d(raw + (size_t)tid * K::kRawSlot, tmap, base, kGroup ? 0 : slice0, a.row0 + it, &raw_bar);
+        tma_load_3d(raw + (size_t)tid * K::kRawSlot, tmap, base, kGroup ? 0 : slice0, kSplit ? a.row0 + it : it,
+                    &raw_bar);
       } else {
         mbar_arrive(&raw_bar);
       }
@@ -861,7 +862,7 @@ __device__ __forceinline__ void bp_tile(const BPArgs &a, int bx, int by, int bz,
         }
 #pragma unroll
         for (int k = 0; k < S; ++k) {
-          if (k < nsl && a.part) {
+          if (kSplit && k < nsl) {
             a.part[((long long)(slice0 + k) * ncol + y) * ncol + x] = make_float2(sum[b][c][k], comp[b][c][k]);
           } else if (k < nsl) {
             const float v = keep ? __fsub_rn(sum[b][c][k], comp[b][c][k]) * a.scale : 0.f;
@@ -873,32 +874,41 @@ __device__ __forceinline__ void bp_tile(const BPArgs &a, int bx, int by, int bz,
   }
 }
 
-template <typename T, int S, bool kPerAngleKahan, int V, bool kGroup = false>
+// kSplit: angle groups.  A kernel of its own: the group's rows, samples and angles
+// are then the CTA's, where the unsplit kernel reads the launch's from the constant
+// bank (with one kernel for both the unsplit launches took 1-5 % longer, up to 23 %
+// with 16-bit samples in rows that are not 16-byte aligned).
+template <typename T, int S, bool kPerAngleKahan, int V, bool kGroup = false, bool kSplit = false>
 __global__ void __launch_bounds__(BPCfg<T, S, V>::kThreads, BPCfg<T, S, V>::kMinBlocks)
-    bp_kernel(BPArgs a, const __grid_constant__ CUtensorMap tmap) {
+    bp_kernel(BPArgs args, const __grid_constant__ CUtensorMap tmap) {
   using K = BPCfg<T, S, V>;
   extern __shared__ __align__(16) unsigned char smem[];
-  if (a.gate) {
-    const bool left = atb::bp_left_to_gather(a.gate, a.ngate, a.nrow);
-    if (!left && (a.interior < 0.0 || atb::bp_interior(blockIdx.x * K::TX, blockIdx.y * K::TY, a.ncol, a.interior)))
-      return;
-  }
-  int bz = blockIdx.z;
-  if (a.part) {  // this CTA's angle group
-    const int nz = gridDim.z / a.ngroup, g = bz / nz;
-    bz -= g * nz;
+  if constexpr (kSplit) {
+    BPArgs a = args;
+    const int nz = gridDim.z / a.ngroup, g = blockIdx.z / nz;
     a.row0 = g * a.group_rows;
     a.sino = reinterpret_cast<const T *>(a.sino) + a.row0 * a.srs;
     a.trig += a.row0;
     a.nrow = min(a.group_rows, a.nrow - a.row0);
     a.part += (long long)g * a.nslice * ncol2(a.ncol);
-  }
-  if constexpr (kPerAngleKahan) {
-    bp_tile<T, S, true, V, kGroup>(a, blockIdx.x, blockIdx.y, bz, smem, 0u, &tmap);
-  } else {
     __shared__ uint32_t tmem_slot;
     const uint32_t tmem = tmem_alloc_cta<K::kTmemCols>(&tmem_slot);
-    bp_tile<T, S, false, V, kGroup>(a, blockIdx.x, blockIdx.y, bz, smem, tmem, &tmap);
+    bp_tile<T, S, false, V, false, true>(a, blockIdx.x, blockIdx.y, blockIdx.z - g * nz, smem, tmem, &tmap);
+    tmem_free_cta<K::kTmemCols>(tmem);
+    return;
+  }
+  if (args.gate) {
+    const bool left = atb::bp_left_to_gather(args.gate, args.ngate, args.nrow);
+    if (!left && (args.interior < 0.0 ||
+                  atb::bp_interior(blockIdx.x * K::TX, blockIdx.y * K::TY, args.ncol, args.interior)))
+      return;
+  }
+  if constexpr (kPerAngleKahan) {
+    bp_tile<T, S, true, V, kGroup>(args, blockIdx.x, blockIdx.y, blockIdx.z, smem, 0u, &tmap);
+  } else if constexpr (!kSplit) {
+    __shared__ uint32_t tmem_slot;
+    const uint32_t tmem = tmem_alloc_cta<K::kTmemCols>(&tmem_slot);
+    bp_tile<T, S, false, V, kGroup>(args, blockIdx.x, blockIdx.y, blockIdx.z, smem, tmem, &tmap);
     tmem_free_cta<K::kTmemCols>(tmem);
   }
 }
@@ -1094,8 +1104,6 @@ template <typename T, int S, bool kPerAngleKahan, int V = 0, bool kGroup = false
 int launch_bp(BPArgs a, int nslices, cudaStream_t st, float2 *work = nullptr) {
   using K = BPCfg<T, S, V>;
   auto fn = bp_kernel<T, S, kPerAngleKahan, V, kGroup>;
-  const int rc = atb::ensure_smem(fn, K::kSmem, "atb_backproject", K::kThreads, kPerAngleKahan ? 0 : K::kTmemCols);
-  if (rc != ATB_OK) return rc;
   CUtensorMap map;
   std::memset(&map, 0, sizeof(map));
   // TMA staging for 2- and 4-slice CTAs (a 4-slice stack of 2560 x 1801
@@ -1109,6 +1117,7 @@ int launch_bp(BPArgs a, int nslices, cudaStream_t st, float2 *work = nullptr) {
   if (work) {
     const int rows = group_rows<T, S, V>(a.nrow, nslices, a.ncol);
     if (rows < a.nrow) {
+      if constexpr (!kPerAngleKahan && !kGroup) fn = bp_kernel<T, S, false, V, false, true>;
       a.group_rows = rows;
       a.ngroup = (a.nrow + rows - 1) / rows;
       a.part = work;
@@ -1121,6 +1130,8 @@ int launch_bp(BPArgs a, int nslices, cudaStream_t st, float2 *work = nullptr) {
       grid.z *= a.ngroup;
     }
   }
+  const int rc = atb::ensure_smem(fn, K::kSmem, "atb_backproject", K::kThreads, kPerAngleKahan ? 0 : K::kTmemCols);
+  if (rc != ATB_OK) return rc;
   fn<<<grid, K::kThreads, K::kSmem, st>>>(a, map);
   const int rcl = atb::check_launch("atb_backproject");
   if (rcl != ATB_OK || !a.part) return rcl;
