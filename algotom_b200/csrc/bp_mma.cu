@@ -827,7 +827,7 @@ int launch_mma(const MmaArgs &a, const CUtensorMap &map, cudaStream_t st) {
 // 1.4e-7 of an image, after 8 0.7e-7 (half of it at 200 pixels).  The gather
 // kernel's error, from its positions, falls as the angles and grows with the
 // image, 2.2e-7 (ncol / 1024) sqrt(901 / nrow), so that 16 angles are the less
-// exact choice from nrow = ncol^2 / 1100 on.  Errors of filtered sinograms
+// exact choice from nrow = ncol^2 / 450 on.  Errors of filtered sinograms
 // against FP64 with 16 angles, with 8, and with the gather kernel (1e-8):
 //   901 x 200: 10.1, 3.8, 6.5;  901 x 512: 13.6, 6.2, 12.0;  901 x 1024: 14.1,
 //   7.8, 22.5;  1801 x 320: 11.8, 4.9, 6.2;  1801 x 720: 13.8, 6.5, 11.6
@@ -836,7 +836,7 @@ int launch_mma(const MmaArgs &a, const CUtensorMap &map, cudaStream_t st) {
 // 2-D ramp filter magnifies it: BPF of 901 x 1280 has 4.0e-6 with 8 and 4.1e-6
 // with 16 angles (4.2e-6 with the gather kernel).
 int fold_steps(const MmaArgs &a) {
-  return a.edge_pad || (long long)a.ncol * a.ncol < 600ll * a.nrow ? kFoldShort : kFoldLong;
+  return a.edge_pad || (long long)a.ncol * a.ncol < 500ll * a.nrow ? kFoldShort : kFoldLong;
 }
 
 int launch(const MmaArgs &a, int S, const CUtensorMap &map, cudaStream_t st) {
