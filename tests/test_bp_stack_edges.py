@@ -59,7 +59,8 @@ def _centres(name, t, ang, c0, spacing, n, edge_pad, flags=0):
 @pytest.mark.parametrize("nrow,nslice,ncol,cen", [
     (1, 15, 16, 7.5), (3, 16, 8, 3.0), (4, 17, 15, 9.25), (7, 24, 17, 0.0),
     (8, 25, 31, 30.0), (9, 31, 33, 16.0), (16, 32, 48, 20.75),
-    (17, 33, 40, 19.5), (33, 47, 65, 33.25), (40, 64, 170, 12.125)])
+    (17, 33, 40, 19.5), (33, 47, 65, 33.25), (40, 64, 170, 12.125),
+    (5, 16, 1, 0.0), (6, 16, 2, 0.5), (7, 17, 3, 1.0), (9, 15, 5, 2.25)])
 def test_forced_stack_against_oracle(cuda, nrow, nslice, ncol, cen, edge_pad):
     ang = np.linspace(0.0, np.pi, nrow)
     x = _stack(nrow, nslice, ncol)
