@@ -1054,17 +1054,23 @@ __global__ void __launch_bounds__(256) sum_groups_kernel(BPArgs a) {
 // A group costs its partial image, whatever its angles, and earns a share of the
 // time that CTAs would stand idle in (mostly the last wave), so that few angles
 // bear few groups or none: at most a group for each angle times (0.1 idle share +
-// 0.005), 0.01 for the larger tiles, whose CTAs end unevenly.  Times without, with
-// the groups above alone, and with this rule (no mask):
+// 0.005), 0.01 for the larger tiles, whose CTAs end unevenly, and 64 angles (120
+// with edge padding) for the launch and the scratch of a call.  Times without, with the groups above alone,
+// and with this rule (no mask):
 //   one slice    120 x 1024: 82, 91, 82; 361 x 1024: 243, 217, 217; 181 x 2560:
 //                440, 527, 440; 720 x 2560: 1688, 1655, 1655
 //   two          120 x 1024: 125, 181, 125; 361 x 1024: 350, 361, 339; 181 x 1536:
 //                342, 392, 342
 //   four, eight  181 x 800: 259, 210, 206; 65 x 1024: 113, 147, 113; 65 x 640 (8):
 //                111, 138, 111
-// Of 780 combinations none is over 1.07 of the better of the first two.
+// Of 780 combinations none of 120 angles and more is over 1.05 of the better of the
+// first two.  With edge padding there is no checked path, and both sides differ:
+//   one slice, 64 x 64   361 x 800: 151, 142 (32 x 32), 103 (6); 720 x 1024: 291,
+//                        382 (32 x 32), 265 (5); 181 x 1024: 79, 113 (32 x 32), 85 (2)
+//   two                  720 x 1300: 920, 969 (5), 946 (2); 720 x 1024: 621, 569 (4)
+//   eight                181 x 512: 140, 160 (3); 720 x 512: 523, 507 (7)
 template <typename T, int S, int V>
-int group_rows(int nrow, int nslices, int ncol) {
+int group_rows(int nrow, int nslices, int ncol, bool edge_pad) {
   using K = BPCfg<T, S, V>;
   const long long tiles =
       (long long)((ncol + K::TX - 1) / K::TX) * ((ncol + K::TY - 1) / K::TY) * ((nslices + S - 1) / S);
@@ -1072,36 +1078,65 @@ int group_rows(int nrow, int nslices, int ncol) {
   constexpr long long slots = 148 * K::kMinBlocks;
   const double idle = 1.0 - (double)tiles / (double)((tiles + slots - 1) / slots * slots);
   long long g;
-  double angles_per_tile, base = 0.005;
-  if (S == 1 && V == 1) {
+  double angles_per_tile = 0.36, base = 0.005, share = 0.1, fewest = 3.6;
+  if (S == 1 && edge_pad) {
+    g = tiles > 3000 ? 1 : std::min(16ll, std::max(4ll, 800 / tiles));
+    angles_per_tile = 0.5;
+    fewest = 4.0;
+  } else if (S == 1 && V == 1) {
     g = tiles > 1700 ? 1 : std::min(16ll, std::max(5ll, 11000 / tiles));
-    angles_per_tile = 0.15;
+    angles_per_tile = 0.18;
+    fewest = 3.0;
   } else if (S == 1) {
     g = tiles > 3000 || nrow < 300 ? 1 : std::min(12ll, std::max(6ll, 4500 / tiles));
     angles_per_tile = 0.3;
     base = 0.01;
+    fewest = 3.0;
   } else if (S == 2) {
-    g = tiles > 1500 ? 1 : std::min(10ll, std::max(4ll, 4500 / tiles));
-    angles_per_tile = 0.36;
+    g = tiles > (edge_pad ? 800 : 1500) ? 1 : std::min(10ll, std::max(4ll, 4500 / tiles));
   } else {
     g = tiles > 600 ? 1 : std::min(8ll, 2000 / tiles);
-    angles_per_tile = 0.36;
   }
-  if ((double)nrow < angles_per_tile * (double)tiles) return nrow;
-  g = std::min(g, (long long)((double)nrow * (0.1 * idle + base)));
-  if (g < 3) return nrow;
-  g = std::min(g, (long long)nchunk);
+  if (S >= 2 && edge_pad) {
+    if (tiles > 400) g = std::min(g, 4ll);
+    share = 0.08;
+    base = 0.003;
+  }
+  const double most = (double)nrow * (share * idle + base);
+  if (nrow < (edge_pad ? 120 : 64) || (double)nrow < angles_per_tile * (double)tiles || most < fewest) return nrow;
+  g = std::min(std::min(g, (long long)most), (long long)nchunk);
   return g <= 1 ? nrow : (int)((nchunk + g - 1) / g * K::kChunk);
 }
 // The tile variant of a single slice that may be split: the one that is faster
 // unsplit (900 x 1300: 811 us in 64 x 64 tiles, 751 in 32 x 32 ones; 1200 x 1536:
 // 1155 and 1285).  Split, the larger tiles win from 700 pixels on (900 x 1024:
 // 400 and 446), but their FP32 positions are further from the tile's middle and
-// less exact (5.4e-7 against 4.7e-7 of error at 900 x 1024).
-int split_variant(int ncol) { return ncol < 1400 ? 1 : 0; }
+// less exact (5.4e-7 against 4.7e-7 of error at 900 x 1024).  With edge padding
+// the larger tiles win everywhere (900 x 1024 unsplit: 367 and 469) and are what
+// single slices of BPF have had.
+int split_variant(int ncol, bool edge_pad) { return ncol < 1400 && !edge_pad ? 1 : 0; }
+
+// bytes of the partial images of dispatch's largest launch; 0 without groups.  (By
+// the groups without edge padding: with it a launch has groups where these bytes
+// hold them.)
+template <typename T>
+long long split_bytes(int nrow, int nslice, int ncol) {
+  long long need = 0;
+  auto add = [&](int rows, int n) {
+    const long long groups = (nrow + rows - 1) / rows;
+    if (groups > 1 && groups * n * ncol * (long long)ncol * 8 > need) need = groups * n * ncol * (long long)ncol * 8;
+  };
+  const int n4 = (nslice / 4) * 4, rem = nslice - n4;
+  if (n4 > 0) add(group_rows<T, 4, 0>(nrow, n4, ncol, false), n4);
+  if (rem >= 2) add(group_rows<T, 2, 0>(nrow, 2, ncol, false), 2);
+  if (rem & 1)
+    add(split_variant(ncol, false) ? group_rows<T, 1, 1>(nrow, 1, ncol, false)
+                                   : group_rows<T, 1, 0>(nrow, 1, ncol, false), 1);
+  return need;
+}
 
 template <typename T, int S, bool kPerAngleKahan, int V = 0, bool kGroup = false>
-int launch_bp(BPArgs a, int nslices, cudaStream_t st, float2 *work = nullptr) {
+int launch_bp(BPArgs a, int nslices, cudaStream_t st, float2 *work = nullptr, long long work_bytes = 0) {
   using K = BPCfg<T, S, V>;
   auto fn = bp_kernel<T, S, kPerAngleKahan, V, kGroup>;
   CUtensorMap map;
@@ -1115,11 +1150,12 @@ int launch_bp(BPArgs a, int nslices, cudaStream_t st, float2 *work = nullptr) {
   a.row0 = 0;
   a.part = nullptr;
   if (work) {
-    const int rows = group_rows<T, S, V>(a.nrow, nslices, a.ncol);
-    if (rows < a.nrow) {
+    const int rows = group_rows<T, S, V>(a.nrow, nslices, a.ncol, a.edge_pad);
+    const long long groups = (a.nrow + rows - 1) / rows;
+    if (groups > 1 && groups * nslices * a.ncol * (long long)a.ncol * 8 <= work_bytes) {
       if constexpr (!kPerAngleKahan && !kGroup) fn = bp_kernel<T, S, false, V, false, true>;
       a.group_rows = rows;
-      a.ngroup = (a.nrow + rows - 1) / rows;
+      a.ngroup = (int)groups;
       a.part = work;
       // the partial images hold this launch's slices only
       a.sino = static_cast<const T *>(a.sino) + a.slice_base * a.sss;
@@ -1141,46 +1177,33 @@ int launch_bp(BPArgs a, int nslices, cudaStream_t st, float2 *work = nullptr) {
   return atb::check_launch("atb_backproject (angle groups)");
 }
 
-// work: null, or scratch for the angle groups (split_bytes)
+// work: null, or scratch of split_bytes for the angle groups
 template <typename T>
 int dispatch(BPArgs a, int per_angle_kahan, int variant, cudaStream_t st, float2 *work) {
   if (per_angle_kahan) return launch_bp<T, 1, true>(a, a.nslice, st);
+  const long long bytes = work ? split_bytes<T>(a.nrow, a.nslice, a.ncol) : 0;
   if (work && (a.nslice & 1)) {  // the single slice's tiles where it is split
-    const int v = split_variant(a.ncol);
-    if ((v ? group_rows<T, 1, 1>(a.nrow, 1, a.ncol) : group_rows<T, 1, 0>(a.nrow, 1, a.ncol)) < a.nrow) variant = v;
+    const int v = split_variant(a.ncol, a.edge_pad);
+    if ((v ? group_rows<T, 1, 1>(a.nrow, 1, a.ncol, a.edge_pad) : group_rows<T, 1, 0>(a.nrow, 1, a.ncol, a.edge_pad)) <
+        a.nrow)
+      variant = v;
   }
-  if (a.nslice == 1 && variant == 1) return launch_bp<T, 1, false, 1>(a, 1, st, work);
+  if (a.nslice == 1 && variant == 1) return launch_bp<T, 1, false, 1>(a, 1, st, work, bytes);
   // four slices per CTA for the bulk of a stack, then the remainder
   const int n4 = (a.nslice / 4) * 4;
   int rc = ATB_OK;
-  if (n4 > 0) rc = launch_bp<T, 4, false>(a, n4, st, work);
+  if (n4 > 0) rc = launch_bp<T, 4, false>(a, n4, st, work, bytes);
   if (rc != ATB_OK) return rc;
   const int rem = a.nslice - n4;
   if (rem == 0) return ATB_OK;
   a.slice_base = n4;
   if (rem >= 2) {
-    rc = launch_bp<T, 2, false>(a, 2, st, work);
+    rc = launch_bp<T, 2, false>(a, 2, st, work, bytes);
     if (rc != ATB_OK || rem == 2) return rc;
     a.slice_base = n4 + 2;
   }
-  if (variant == 1) return launch_bp<T, 1, false, 1>(a, 1, st, work);
-  return launch_bp<T, 1, false>(a, 1, st, work);
-}
-
-// bytes of the partial images of dispatch's largest launch; 0 without groups
-template <typename T>
-long long split_bytes(int nrow, int nslice, int ncol) {
-  long long need = 0;
-  auto add = [&](int rows, int n) {
-    const long long groups = (nrow + rows - 1) / rows;
-    if (groups > 1 && groups * n * ncol * (long long)ncol * 8 > need) need = groups * n * ncol * (long long)ncol * 8;
-  };
-  const int n4 = (nslice / 4) * 4, rem = nslice - n4;
-  if (n4 > 0) add(group_rows<T, 4, 0>(nrow, n4, ncol), n4);
-  if (rem >= 2) add(group_rows<T, 2, 0>(nrow, 2, ncol), 2);
-  if (rem & 1)
-    add(split_variant(ncol) ? group_rows<T, 1, 1>(nrow, 1, ncol) : group_rows<T, 1, 0>(nrow, 1, ncol), 1);
-  return need;
+  if (variant == 1) return launch_bp<T, 1, false, 1>(a, 1, st, work, bytes);
+  return launch_bp<T, 1, false>(a, 1, st, work, bytes);
 }
 
 }  // namespace
