@@ -886,7 +886,8 @@ int padded(int n) { return (n + 7) / 8 * 8; }
 // Angles from which a group of n slices is worth its scan, packing and launch
 // (the gather kernel has one launch, of a cost per slice).  Time against the
 // gather kernel's by angles, read off 15 to 32 slices of 32 to 2560 pixels:
-//   up to 160 pixels  16 slices: 1.15 (16), 0.85 (24); 32 slices: 1.07 (24), 0.96 (32)
+//   up to 160 pixels  16 slices: 1.15 (16), 0.85 (24); 32 slices: 1.07 (24), 0.96
+//                     (32); whole calls, with three launches more: 1.2 (33)
 //   24 slices         512: 1.11 (32), 0.95 (48); 1536: 1.08 (48), 0.94 (64)
 //   32                800: 1.06 (24), 1.00 (32), 0.85 (48)
 //   21                1536: 1.03 (64), 0.91 (96); 2560: 1.05 (64), 0.93 (96)
@@ -896,7 +897,7 @@ int padded(int n) { return (n + 7) / 8 * 8; }
 //   15                800: 0.94 (64); 1536: 0.99 (256); 2560: 1.00 (384): the two more
 //                     launches of the gather kernel's remainder weigh less and less
 int fewest_angles(int n, int ncol) {
-  if (ncol <= 160) return n > 16 ? 32 : 24;
+  if (ncol <= 160) return 64;
   if (n >= 18) return n >= 28 ? 48 : n >= 24 ? 56 : n >= 21 ? 72 : 120;
   const int w = ncol < 1536 ? ncol : 1536;
   const int by_size = n == 17 ? 168 * w / 1536 : n == 16 ? 320 * w / 1536 : 320 * w / 1536 * w / 1536;
@@ -1001,17 +1002,17 @@ extern "C" int atb_backproject_stack(const void *sino, int sino_dtype, int64_t s
       first += n;
       return rc;
     };
-    int whole = (nslice - first) / 32 * 32;
-    // (without angle groups one launch gives the same bits)
-    const bool split = next_group(sino_dtype, nrow, ncol, 32) == 0 && atb::bp_gather_workspace(nrow, 32, ncol) > 0;
-    while (whole > 0) {
-      const int n = split ? 32 : whole;
-      const int rc = gather(n, split);
+    const auto groups = [&](int n) {
+      return n > 0 && next_group(sino_dtype, nrow, ncol, n) == 0 && atb::bp_gather_workspace(nrow, n, ncol) > 0;
+    };
+    const int left = (nslice - first) % 32;
+    const bool split = groups(32), split_left = groups(left);
+    if (!split && !split_left) return gather(nslice - first, false);  // (one launch has the same bits)
+    while (nslice - first > left) {
+      const int rc = gather(split ? 32 : nslice - first - left, split);
       if (rc != ATB_OK) return rc;
-      whole -= n;
     }
-    const int left = nslice - first;
-    return left ? gather(left, next_group(sino_dtype, nrow, ncol, left) == 0) : ATB_OK;
+    return left ? gather(left, split_left) : ATB_OK;
   }
   return atb::bp_gather(sino, sino_dtype, sino_row_stride, sino_slice_stride, nrow, nslice, ncol, trig, center, edge_pad,
                         mask_r2, scale, out, out_row_stride, out_slice_stride, flags, nullptr, nullptr, stream);

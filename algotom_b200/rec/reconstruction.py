@@ -184,7 +184,8 @@ def backproject(sino3, angles, center, edge_pad=False, mask_r2=-1.0,
     if out is None:
         out = torch.empty((ncol, nslice, ncol), dtype=torch.float32,
                           device=dev)
-    if kahan != "angle" and variant is None:
+    # (no rule of the entry point takes fewer angles anywhere)
+    if kahan != "angle" and variant is None and nrow >= 24:
         need = _stack_need(code, nrow, nslice, ncol)
         if need > 0:
             ws = _stack_workspace(need, dev)

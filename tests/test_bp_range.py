@@ -15,7 +15,7 @@ from algotom_b200.rec import reconstruction as R
 from oracle import fbp_oracle as O
 
 pytestmark = pytest.mark.gpu
-NROW, NCOL, CEN = 61, 97, 47.3
+NROW, NCOL, CEN = 101, 97, 47.3
 ANG = np.linspace(0.0, np.pi, NROW)
 
 

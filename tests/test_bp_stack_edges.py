@@ -89,11 +89,11 @@ def test_forced_centres_against_oracle(cuda, n, spacing, c0, edge_pad):
 
 
 @pytest.mark.parametrize("nrow,nslice,ncol,tensor", [
-    (23, 16, 100, 0), (24, 16, 100, 16), (47, 32, 161, 0), (48, 32, 161, 32),
+    (63, 16, 100, 0), (64, 16, 100, 16), (47, 32, 161, 0), (48, 32, 161, 32),
     (56, 24, 161, 24), (71, 21, 200, 0), (72, 21, 200, 21), (119, 18, 200, 0),
     (120, 18, 200, 18), (65, 16, 320, 0), (66, 16, 320, 16),
     (34, 15, 512, 0), (35, 15, 512, 15), (55, 24, 161, 0),
-    (31, 17, 100, 0), (32, 17, 100, 17), (50, 47, 1000, 32)])
+    (63, 17, 160, 0), (64, 17, 160, 17), (50, 47, 1000, 32)])
 def test_groups_with_few_angles_take_the_gather_kernel(cuda, nrow, nslice,
                                                        ncol, tensor):
     """The first ``tensor`` slices run on the tensor cores, whose bits do not

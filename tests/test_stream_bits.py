@@ -31,8 +31,8 @@ def test_groups_cover_the_spans(nslice, nrow, ncol, storage, kahan, joined):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("nslice,nrow,ncol,storage,kahan", [
-    (128, 91, 96, "float32", "chunk"), (138, 91, 200, "float32", "chunk"),
-    (144, 64, 64, "float16", "chunk"), (134, 20, 170, "float32", "chunk"),
+    (128, 101, 96, "float32", "chunk"), (138, 91, 200, "float32", "chunk"),
+    (144, 100, 64, "float16", "chunk"), (134, 20, 170, "float32", "chunk"),
     (134, 181, 64, "bfloat16", "chunk"), (70, 181, 128, "bfloat16", "chunk"),
     (132, 61, 64, "float32", "angle"), (38, 2100, 48, "float32", "chunk")])
 def test_streamed_bits_are_the_resident_ones(cuda, nslice, nrow, ncol,
