@@ -431,7 +431,8 @@ def run_ours(args, rank, world, local_rank):
     if rank != 0:
         return
 
-    # ---- accuracy of slice 0 against the FP64 oracle; CPU baseline
+    # ---- accuracy of slice 0 (of a launch of 32 on the tensor cores, as the
+    # timed ones) against the FP64 oracle; CPU baseline
     err = None
     cpu = None
     if not args.no_oracle:
@@ -484,17 +485,22 @@ def run_ours(args, rank, world, local_rank):
                    "l2": "inputs larger than L2 (4.7 GB sinogram per GPU)"},
         "slices_per_s": world * nslice * args.steps / t_dev,
         "accuracy": err,
-        "roofline": {"bound": "tensor", "kernel": "bp_mma_kernel",
+        # bound by the issue of the weight rows; the figure is the tensor pipe's
+        # share: every product of its tiles, of whose 16 weights a row 14 are
+        # structural zeros, times the split's four terms
+        "roofline": {"bound": "issue", "kernel": "bp_mma_kernel",
                      "achieved": tensor_achieved, "peak": tensor_peak,
                      "unit": "TFLOP/s", "frac": tensor_achieved / tensor_peak,
                      "traffic": (tpu * bp_upd if tpu else None),
                      "flop_per_update": MMA_FLOP_PER_UPDATE,
+                     "useful_flop_per_update": FLOP_PER_UPDATE,
                      "live_fraction": live,
                      "updates_per_s": bp_upd / t_bp,
                      "ms_per_launch": t_bp * 1e3,
                      "peak_source": "float16 tensor cores, the measured bf16 "
-                                    "GEMM burst (%s); regions outside the "
-                                    "circle mask do no products" % src,
+                                    "GEMM burst (%s); zero weights counted, "
+                                    "regions outside the circle mask, which "
+                                    "do no products, not" % src,
                      "traffic_source": ("ncu dram__bytes_read.sum + "
                                         "dram__bytes_write.sum per update "
                                         "from %s (%s), times this launch's "
@@ -570,7 +576,16 @@ def batch_measure(n_items=64, steps=3, warmup=3, check=True):
     peaks, src = _peaks()
     f_clk = float(peaks.get("sm_max_mhz", 1965.0)) * 1e6
     smem_peak = SMEM_BYTES_PER_CLK_PER_SM * N_SM * f_clk / 1e9
-    smem_achieved = SMEM_BYTES_PER_UPDATE * bf.updates / t_bp / 1e9
+    # updates of the tiles that the circle masks leave; the others read nothing
+    tile = 32 if bf.variant == 1 else 64
+    live = 0.0
+    for g in geo:
+        edge = np.arange(0, g["ncol"], tile) - g["ncol"] // 2
+        near = np.maximum(0, np.maximum(edge, -(edge + tile - 1)))
+        r2 = R._mask_r2(1.0, g["center"], g["ncol"])
+        live += g["nrow"] * g["ncol"] ** 2 * float(
+            np.mean(near[:, None] ** 2 + near[None] ** 2 <= r2))
+    smem_achieved = SMEM_BYTES_PER_UPDATE * live / t_bp / 1e9
     err = None
     if check:
         from oracle import fbp_oracle as O
@@ -597,6 +612,7 @@ def batch_measure(n_items=64, steps=3, warmup=3, check=True):
                      "achieved": smem_achieved, "peak": smem_peak,
                      "unit": "GB/s", "frac": smem_achieved / smem_peak,
                      "bytes_per_update": SMEM_BYTES_PER_UPDATE,
+                     "live_fraction": live / bf.updates,
                      "updates_per_s": bf.updates / t_bp,
                      "ms_per_launch": t_bp * 1e3,
                      "peak_source": "shared-memory delivery, 128 B/clk x 148 "
