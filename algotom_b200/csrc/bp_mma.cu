@@ -50,14 +50,13 @@
 // - four warps read each tile's sums, zero them and keep the compensated
 //   totals, in registers that the other warps give up.
 // The tiles' sums end in turn, so that one tile's read is covered by the
-// others' MMAs.  What bounds it: the weight warps' issue (72 % of all issue slots
-// taken, the integer pipe 57 %), which is why the cost of a launch hardly depends
-// on the number of slices; the tensor cores are busy 45 % of the time.  Under
+// others' MMAs.  What bounds it: the weight warps' issue (69 % of all issue slots
+// taken, the integer pipe 58 %), which is why the cost of a launch hardly depends
+// on the number of slices; the tensor cores are busy 46 % of the time.  Under
 // sustained load the power cap sets the clock (1.70 GHz).
-// Measured, 1801 angles of 2560 bins, 32 slices, no mask: 53.9 ms against
-// 100.5 ms with the gather kernel (7.0e12 and 3.8e12 updates/s); 901 x 1024: 4.14
-// against 8.68; 901 x 1280: 6.16 against 10.03 ms with 24 slices, 6.23 against
-// 6.76 with 16.
+// Measured, 1801 angles of 2560 bins, 32 slices, no mask: 55.7 ms against
+// 100.5 ms with the gather kernel (6.8e12 and 3.8e12 updates/s); 901 x 1280: 6.0
+// against 10.0 ms with 24 slices, 5.4 against 6.8 with 16.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -831,7 +830,7 @@ int launch_mma(const MmaArgs &a, const CUtensorMap &map, cudaStream_t st) {
 // against FP64 with 16 angles, with 8, and with the gather kernel (1e-8):
 //   901 x 200: 10.1, 3.8, 6.5;  901 x 512: 13.6, 6.2, 12.0;  901 x 1024: 14.1,
 //   7.8, 22.5;  1801 x 320: 11.8, 4.9, 6.2;  1801 x 720: 13.8, 6.5, 11.6
-// 8 angles cost 1801 x 2560 with 32 slices 59.4 ms instead of 55.7.  With edge
+// 8 angles cost 1801 x 2560 with 32 slices 59.1 ms instead of 56.1.  With edge
 // padding (BPF) the samples have one sign, so that the bias is the larger, and the
 // 2-D ramp filter magnifies it: BPF of 901 x 1280 has 4.0e-6 with 8 and 4.1e-6
 // with 16 angles (4.2e-6 with the gather kernel).
@@ -868,8 +867,9 @@ int prepare(const void *sino, long long srs, long long sss, int nrow, int nsl, i
 
 // slices of the next launch of a stack with n left: 0 if the gather kernel is
 // the faster one for all of them.  A launch costs the same for 16 as for 10
-// slices, at 901 x 1280 6.1 ms, and the gather kernel 0.43 ms per slice: 6.0
-// for 14, 6.5 for 15.  bfloat16 samples stay with the gather kernel, whose
+// slices, at 901 x 1280 5.4 ms, and the gather kernel 0.43 ms per slice, 6.0 for
+// 14; but at 2560 pixels and fewer angles the two meet at 15 and 16
+// (fewest_angles).  bfloat16 samples stay with the gather kernel, whose
 // interpolation differences are bfloat16 too: a user's results would move by
 // that rounding (2e-4) for a faster kernel.  So do stacks of more angles than the
 // truncations bear, whose sums the gather kernel, averaging over its positions'
